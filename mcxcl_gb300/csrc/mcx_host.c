@@ -1271,10 +1271,15 @@ int mcx_rand_blocks(unsigned int seed, uint64_t skip, uint32_t nblock, uint32_t 
 
 /* The field accumulator's fixed-point unit 2^-S (the transport kernel's
    deposits split into int64 counts of 2^-S and float remainders): the
-   largest S, at most 40, for which no element can reach 2^61 counts.  An
+   largest S, at most 40, for which no element can reach 2^62 counts.  An
    element gathers at most every photon's whole path -- the time window at
    the speed of light, in voxels -- times its weight (a replay: the largest
-   replay weight), with a factor 4 to spare. */
+   replay weight), with a factor 4 to spare.  Where photons only lose weight
+   (labels, real weights, no roulette) a photon also leaves no more than its
+   launch weight as energy, or that over the least mua as flux, in all
+   elements together (a factor 2 to spare).  The larger S is worth having: a
+   deposit of 2^(23-S) or more is a whole number of units, so its remainder
+   is exactly zero and the second of its two atomics is not issued. */
 static void field_scale(const Config* cfg, int replay, float* sc, float* unit) {
     const double twin1 = (double)cfg->tstart + (double)cfg->tstep * cfg->maxgate;
     double path = twin1 * 2.99792458e11 / (cfg->unitinmm > 0.f ? cfg->unitinmm : 1.f);
@@ -1286,8 +1291,26 @@ static void field_scale(const Config* cfg, int replay, float* sc, float* unit) {
             wmax = w > wmax ? w : wmax;
         }
     }
-    const double bound = 4.0 * (double)(cfg->nphoton ? cfg->nphoton : 1) * path * wmax;
-    int S = (int)floor(61.0 - log2(bound));
+    double each = 4.0 * path * wmax;
+    if (!replay && cfg->mediabyte <= 4 && !(cfg->omega > 0.f) && !(cfg->minenergy > 0.f) && cfg->outputtype != otL) {
+        double loss = fabs((double)cfg->srcpos.w);
+        for (unsigned int i = 0; i < cfg->extrasrclen; i++) {
+            loss = fmax(loss, fabs((double)cfg->srcdata[i].srcpos.w));
+        }
+        if (cfg->srctype == MCX_SRC_PATTERN || cfg->srctype == MCX_SRC_PATTERN3D) {
+            loss = INFINITY;             /* the pattern's values scale the weight: the path bound stands */
+        }
+        loss = fmax(loss, 1.0);
+        double mua = INFINITY;
+        for (unsigned int i = 1; i < cfg->medianum; i++) {
+            mua = fmin(mua, (double)cfg->prop[i].mua);
+        }
+        /* the saved reflectance deposits the weight itself */
+        const double most = cfg->outputtype == otEnergy ? loss : (mua > 0.0 ? loss * fmax(1.0, 1.0 / mua) : INFINITY);
+        each = fmin(each, 2.0 * most);
+    }
+    const double bound = (double)(cfg->nphoton ? cfg->nphoton : 1) * each;
+    int S = (int)floor(62.0 - log2(bound));
     S = S < 0 ? 0 : (S > 40 ? 40 : S);
     *sc = ldexpf(1.f, S);
     *unit = ldexpf(1.f, -S);
