@@ -25,6 +25,7 @@ NVCC_COMMON = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC", "-I" + C
 # 512-simulation batch 8 % faster)
 UNITS = {
     "mcx_kernel_fast.cu": ["--use_fast_math", "-Xptxas", "--register-usage-level=2"],
+    "mcx_kernel_label.cu": ["--use_fast_math", "-Xptxas", "--register-usage-level=2"],
     "mcx_kernel_batch.cu": ["--use_fast_math", "-Xptxas", "--register-usage-level=2"],
     "mcx_kernel_exact.cu": ["-fmad=false", "-prec-div=true", "-prec-sqrt=true", "-ftz=false"],
     "mcx_device.cu": [],

@@ -38,7 +38,7 @@ struct mcxg_session {
     mcxg_kparams kp{};
     bool has_problem = false;
     bool has_seeds = false;
-    bool up_fast = false, up_exact = false;
+    bool up_fast = false, up_exact = false, up_label = false;
 
     void* d_media = nullptr;
     size_t media_cap = 0;
@@ -477,6 +477,25 @@ size_t shared_bytes(const mcxg_kparams& kp, int block) {
     return (size_t)kp.medianum * 32 + (size_t)block * 32 + (size_t)(kp.nphase + kp.nangle) * 4 + det * (size_t)block * 4;
 }
 
+/* the configurations of mcx_transport_label beyond what the common
+   instantiations fix: one byte a voxel, one source, launched photons that
+   deposit flux, fluence or energy, no scattering count at which g drops to 0
+   (a float count of scatterings stops below 2^24 + 1), 15-bit voxel indices */
+bool label_config(const mcxg_kparams& kp) {
+    return kp.mediaword == 1 && !kp.replay && kp.save2pt && !kp.extrasrclen && kp.gscatter > (1u << 24) &&
+           (kp.outputtype == otFlux || kp.outputtype == otFluence || kp.outputtype == otEnergy ||
+            kp.outputtype >= otAdjoint) &&
+           kp.dimx < 32768u && kp.dimy < 32768u && kp.dimz < 32768u;
+}
+
+/* its shared memory: 32 B of launch-time state a thread, three property rows
+   a medium, the detector partial data (a slot for each label and kind), the
+   launch angle table */
+size_t label_shared_bytes(const mcxg_kparams& kp) {
+    const size_t kinds = kp.savedet && kp.maxmedia ? kp.partialdata / kp.maxmedia : 0;
+    return (size_t)mcxg::kLabelBlock * 32 + (size_t)kp.medianum * 48 + kinds * kp.medianum * mcxg::kLabelBlock * 4 + (size_t)kp.nangle * 4;
+}
+
 /* q = umulhi(n, m) >> sh equals n / d for every n < bound: m = ceil(2^(32+sh) / d)
    with the largest sh that keeps m below 2^32, exact when (bound - 1) e <
    2^(32+sh), e = m d - 2^(32+sh) (the rounding error of m times d) */
@@ -885,7 +904,7 @@ int mcxg_set_problem(mcxg_session* s, const void* kparams, size_t kparams_size, 
     }
     s->h_det.assign(detpos ? detpos : prop, detpos ? detpos + 4 * kp.detnum : prop);
     s->h_srcx.assign(srcextra ? srcextra : prop, srcextra ? srcextra + 16 * kp.extrasrclen : prop);
-    s->up_fast = s->up_exact = false;
+    s->up_fast = s->up_exact = s->up_label = false;
     s->has_problem = true;
     s->npol = 0;
     s->tuned = 0;
@@ -911,7 +930,7 @@ int mcxg_set_params(mcxg_session* s, const void* kparams, size_t kparams_size) {
     s->kp = kp;
     s->kp.mediaword = mw;
     s->kp.npattern = np;
-    s->up_fast = s->up_exact = false;
+    s->up_fast = s->up_exact = s->up_label = false;
     return MCXG_OK;
 }
 
@@ -1261,10 +1280,6 @@ int mcxg_simulate(mcxg_session* s, unsigned int flags, float* kernel_ms) {
         MCXG_TRY(mcxg::exact_upload(&kp, s->h_det.data(), kp.detnum, s->h_srcx.data(), kp.extrasrclen, s->st));
         s->up_exact = true;
     }
-    if (!exact && !s->up_fast) {
-        MCXG_TRY(mcxg::fast_upload(&kp, s->h_det.data(), kp.detnum, s->h_srcx.data(), kp.extrasrclen, s->st));
-        s->up_fast = true;
-    }
     {
         /* a run that turns on the complex field after mcxg_set_problem */
         const size_t need = kFieldPlanes * (size_t)kp.fieldlen * field_comps(kp);
@@ -1405,6 +1420,21 @@ int mcxg_simulate(mcxg_session* s, unsigned int flags, float* kernel_ms) {
             s->tile_used = t;
         }
     }
+    /* byte-label volumes in the usual configuration have a kernel of their own */
+    const bool label = !exact && common && label_config(kp) && block == mcxg::kLabelBlock &&
+                       !(lflags & (mcxg::LF_WAGG | mcxg::LF_TILE | mcxg::LF_ACC64 | mcxg::LF_ADJ));
+    if (label) {
+        lflags |= (int)(kp.savedetflag & 0xEu) << mcxg::LF_KINDS;
+        smem = label_shared_bytes(kp);
+    }
+    if (label && !s->up_label) {
+        MCXG_TRY(mcxg::label_upload(&kp, s->h_det.data(), kp.detnum, s->st));
+        s->up_label = true;
+    }
+    if (!exact && !label && !s->up_fast) {
+        MCXG_TRY(mcxg::fast_upload(&kp, s->h_det.data(), kp.detnum, s->h_srcx.data(), kp.extrasrclen, s->st));
+        s->up_fast = true;
+    }
     if (smem > s->info.sharedmem_per_block) {
         return MCXG_ERR_LIMIT;
     }
@@ -1412,7 +1442,7 @@ int mcxg_simulate(mcxg_session* s, unsigned int flags, float* kernel_ms) {
     if (!exact) {
         /* never more blocks than fit at once: a persistent grid must be resident */
         int occ = 0;
-        MCXG_TRY(mcxg::fast_occupancy(lflags, block, smem, &occ));
+        MCXG_TRY(label ? mcxg::label_occupancy(lflags, block, smem, &occ) : mcxg::fast_occupancy(lflags, block, smem, &occ));
         if (occ >= 1 && bpsm > occ) {
             bpsm = occ;
         }
@@ -1425,7 +1455,7 @@ int mcxg_simulate(mcxg_session* s, unsigned int flags, float* kernel_ms) {
     s->block = block;
     if (!exact) {
         cudaFuncAttributes fa;
-        if (mcxg::fast_attributes(lflags, &fa) == cudaSuccess) {
+        if ((label ? mcxg::label_attributes(lflags, &fa) : mcxg::fast_attributes(lflags, &fa)) == cudaSuccess) {
             s->regs = fa.numRegs;
         }
     }
@@ -1436,6 +1466,8 @@ int mcxg_simulate(mcxg_session* s, unsigned int flags, float* kernel_ms) {
         MCXG_TRY(mcxg::exact_rngdump(a, s->info.sm * 4, 256, s->st));
     } else if (exact) {
         MCXG_TRY(mcxg::exact_launch(a, lflags, grid, block, smem, s->st));
+    } else if (label) {
+        MCXG_TRY(mcxg::label_launch(a, lflags, grid, block, smem, s->st));
     } else {
         MCXG_TRY(mcxg::fast_launch(a, lflags, grid, block, smem, s->st));
     }
@@ -1467,7 +1499,7 @@ int mcxg_autotune(mcxg_session* s, uint32_t sample_photons, int* block, int* blo
         samp.oddphoton = (int)(sample_photons - samp.threadphoton * full.nthread);
     }
     s->kp = samp;
-    s->up_fast = false;
+    s->up_fast = s->up_label = false;
     /* the block sizes 64, 128 and 256 at 1,024 resident threads per SM (64
        registers) and 128 and 256 at 512 (uncapped registers), direct
        deposits; then the fastest with warp-aggregated deposits */
@@ -1500,7 +1532,7 @@ int mcxg_autotune(mcxg_session* s, uint32_t sample_photons, int* block, int* blo
         }
     }
     s->kp = full;
-    s->up_fast = false;
+    s->up_fast = s->up_label = false;
     s->block_req = keep_block;
     s->bpsm_req = keep_bpsm;
     if (rc) {
@@ -2105,7 +2137,7 @@ int mcxg_batch_simulate(mcxg_session* s, unsigned int flags, float* kernel_ms) {
     const int bpsm_req = verify ? 3 : (s->bpsm_req ? s->bpsm_req : 4);
     int lflags = (refl ? mcxg::LF_REFL : 0) | (agg ? mcxg::LF_WAGG : 0) | (bpsm_req >= 3 ? mcxg::LF_CAPPED : 0) |
                  (common && !(flags & MCXG_GENERAL) ? mcxg::LF_COMMON : 0) | (verify ? mcxg::LF_ACC64 : 0);
-    int block = s->block_req ? s->block_req : 256;
+    const int block = s->block_req ? s->block_req : 256;
     int occ = 0;
     MCXG_TRY(mcxg::batch_occupancy(lflags, block, (size_t)block * 32, &occ));
     int bpsm = std::max(1, std::min(bpsm_req, occ > 0 ? occ : bpsm_req));

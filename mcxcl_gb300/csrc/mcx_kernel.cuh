@@ -1060,20 +1060,17 @@ __device__ __forceinline__ void save_traj(const KArgs& a, const mcxg_kparams& c_
 }
 
 /*
- * launchnewphoton (mcx_core.cl:1463-2275): close the current photon (escaped
- * weight, saved reflectance, detection) and launch the next one of this
- * reference thread.  Returns 0 on launch, 1 when the thread's quota is done,
- * -1 when no launch position was found.
+ * launchnewphoton (mcx_core.cl:1463-2275), in two parts.  closephoton: the
+ * current photon's escaped weight, saved reflectance and detection; 1 when
+ * the reference thread's quota is done (or the record buffer is full and the
+ * run stops there), else 0.  startphoton: the thread's next photon; 0 on
+ * launch, 1 when a replay has no photon for it, -1 when no launch position
+ * was found.
  */
-template <bool EXACT, bool DET, bool RF, bool POL, bool SVMC, class PS>
-__device__ int launchnewphoton(const KArgs& a, const PS& ps, const Shared& S, Photon& s, unsigned int isdet,
-                               unsigned int vt, unsigned long long* nfailed) {
+template <bool DET, bool POL, bool SVMC, class PS>
+__device__ __forceinline__ int closephoton(const KArgs& a, const PS& ps, const Shared& S, Photon& s, unsigned int isdet,
+                                           unsigned int vt) {
     const mcxg_kparams& c_p = ps.p();
-    const float4* c_srcx = ps.srcx();
-    typedef Mth<EXACT> M;
-    s.w0 = 1.f;
-    s.Lmove = -1.f;
-
     if (DET && c_p.savedet == 3 && *(volatile unsigned int*)a.detcount >= c_p.maxdetphoton) {
         return 1;
     }
@@ -1103,14 +1100,21 @@ __device__ int launchnewphoton(const KArgs& a, const PS& ps, const Shared& S, Ph
             savedetphoton<POL>(a, ps, S, s, isdet);
         }
     }
+    return s.f.w >= (float)(c_p.threadphoton + (vt < (unsigned int)c_p.oddphoton));
+}
+
+template <bool EXACT, bool DET, bool RF, bool POL, bool SVMC, class PS>
+__device__ __forceinline__ int startphoton(const KArgs& a, const PS& ps, const Shared& S, Photon& s, unsigned int vt,
+                                           unsigned long long* nfailed) {
+    const mcxg_kparams& c_p = ps.p();
+    const float4* c_srcx = ps.srcx();
+    typedef Mth<EXACT> M;
+    s.w0 = 1.f;
+    s.Lmove = -1.f;
     if (DET) {
         for (unsigned int i = 0; i < c_p.partialdata; i++) {
             ps.pp(i) = 0.f;
         }
-    }
-
-    if (s.f.w >= (float)(c_p.threadphoton + (vt < (unsigned int)c_p.oddphoton))) {
-        return 1;
     }
 
     if (c_p.replay) {
@@ -1528,6 +1532,15 @@ __device__ int launchnewphoton(const KArgs& a, const PS& ps, const Shared& S, Ph
         ps.pp(c_p.partialdata + 1) = rs;
     }
     return 0;
+}
+
+template <bool EXACT, bool DET, bool RF, bool POL, bool SVMC, class PS>
+__device__ __forceinline__ int launchnewphoton(const KArgs& a, const PS& ps, const Shared& S, Photon& s, unsigned int isdet,
+                                               unsigned int vt, unsigned long long* nfailed) {
+    if (closephoton<DET, POL, SVMC>(a, ps, S, s, isdet, vt)) {
+        return 1;
+    }
+    return startphoton<EXACT, DET, RF, POL, SVMC>(a, ps, S, s, vt, nfailed);
 }
 
 /* ------------------------------------------------------------------ kernel */

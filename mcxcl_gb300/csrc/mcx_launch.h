@@ -87,7 +87,8 @@ struct KArgs {
 
 /* flag bits for the launch entries */
 enum { LF_DET = 1, LF_REFL = 2, LF_WAGG = 4, LF_CAPPED = 8, LF_XMEDIA = 32, LF_COMMON = 64, LF_RF = 128, LF_POL = 256, LF_SVMC = 512,
-       LF_ACC64 = 1024, LF_ADJ = 2048, LF_TILE = 4096 };
+       LF_ACC64 = 1024, LF_ADJ = 2048, LF_TILE = 4096,
+       LF_KINDS = 16 /* bit position of savedetflag's partial-data bits, for the label kernel */ };
 
 /* fast instantiation: hardware transcendental approximations */
 cudaError_t fast_upload(const mcxg_kparams* p, const float* det4, unsigned int ndet, const float* srcx16,
@@ -95,6 +96,13 @@ cudaError_t fast_upload(const mcxg_kparams* p, const float* det4, unsigned int n
 cudaError_t fast_launch(const KArgs& a, int flags, int grid, int block, size_t smem, cudaStream_t st);
 cudaError_t fast_occupancy(int flags, int block, size_t smem, int* blocks_per_sm);
 cudaError_t fast_attributes(int flags, cudaFuncAttributes* attr);
+
+constexpr int kLabelBlock = 256;   /* its threads a block */
+/* the kernel of byte-label volumes in the usual configuration (one source: no extra-source table) */
+cudaError_t label_upload(const mcxg_kparams* p, const float* det4, unsigned int ndet, cudaStream_t st);
+cudaError_t label_launch(const KArgs& a, int flags, int grid, int block, size_t smem, cudaStream_t st);
+cudaError_t label_occupancy(int flags, int block, size_t smem, int* blocks_per_sm);
+cudaError_t label_attributes(int flags, cudaFuncAttributes* attr);
 
 /* exact instantiation: IEEE basic operations only, bit-identical to the oracle */
 cudaError_t exact_upload(const mcxg_kparams* p, const float* det4, unsigned int ndet, const float* srcx16,
