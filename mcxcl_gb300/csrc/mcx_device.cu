@@ -477,6 +477,35 @@ size_t shared_bytes(const mcxg_kparams& kp, int block) {
     return (size_t)kp.medianum * 32 + (size_t)block * 32 + (size_t)(kp.nphase + kp.nangle) * 4 + det * (size_t)block * 4;
 }
 
+/* Blocks per SM (of 256 threads) and lanes per warp for a run of `photons`.
+   A photon takes up to thousands of steps one after another, so a run cannot
+   end before its longest photon, and a step takes the longer the more warps
+   share the SM (cube: 3 us at 32 warps, 0.55 us at a few) and the more lanes
+   of the warp go different ways.  A large run wants all the warps for
+   throughput; one with few photons per SM is faster with fewer.  Kernel times
+   in ms at 4 blocks x 32 lanes and as here: cube 1e4 photons 2.01 -> 1.20,
+   1e5 2.91 -> 1.69, 3e5 3.62 -> 2.37, 1e6 5.93 -> 4.40, 3e6 9.58 -> 8.90;
+   cube + sphere 1e4 2.37 -> 1.95, 1e5 4.48 -> 3.21, 1e6 9.06 -> 7.47; head 1e5
+   2.97 -> 2.92, 1e6 6.81 -> 6.43.  The lines lie where the two shapes beside
+   them measured the same on the three (shapes of 1 to 4 blocks x 2 to 32
+   lanes, 3e3 to 2e7 photons).  The other kernels, with more instructions a
+   step, gain from fewer warps only below 1,000 photons an SM (the replay of
+   9,000 photons 4.7 -> 3.7 ms); at 1e6 photons 2 blocks were 5 to 10 % slower
+   than 4. */
+void shape_for(unsigned long long photons, int sms, bool label, int* blocks, unsigned int* lanes) {
+    const unsigned long long q = photons / (unsigned int)sms;
+    *lanes = 32u;
+    if (q <= 96) {
+        *blocks = 2;
+        *lanes = std::max(1u, (unsigned int)(q + 15) / 16);       /* one photon a lane, over 16 warps */
+    } else if (q <= 1000) {
+        *blocks = 1;
+        *lanes = std::min(32u, (unsigned int)(q + 11) / 12);
+    } else {
+        *blocks = !label ? 4 : (q <= 10000 ? 2 : (q <= 35000 ? 3 : 4));
+    }
+}
+
 /* the configurations of mcx_transport_label beyond what the common
    instantiations fix: one byte a voxel, one source, launched photons that
    deposit flux, fluence or energy, no scattering count at which g drops to 0
@@ -1439,6 +1468,13 @@ int mcxg_simulate(mcxg_session* s, unsigned int flags, float* kernel_ms) {
         return MCXG_ERR_LIMIT;
     }
     int bpsm = exact ? 2 : bpsm_sel;
+    a.lanes = 32;
+    if (!exact && !adjmode && !s->block_req && !s->bpsm_req) {
+        int few = 0;
+        shape_for((unsigned long long)kp.threadphoton * kp.nthread + (unsigned long long)std::max(kp.oddphoton, 0),
+                  s->info.sm, label, &few, &a.lanes);
+        bpsm = std::min(bpsm, few);
+    }
     if (!exact) {
         /* never more blocks than fit at once: a persistent grid must be resident */
         int occ = 0;
@@ -1983,6 +2019,7 @@ int batch_enqueue(mcxg_session* s, int lflags) {
     a.status = s->d_words + 2;
     a.counters = s->d_events;
     a.lo = (unsigned int)s->totalfield;
+    a.lanes = 32;
     if (lflags & mcxg::LF_ACC64) {
         a.acc64 = s->d_acc64;
         a.accf = s->d_accf;

@@ -1725,7 +1725,7 @@ __global__ void __launch_bounds__(256, MINB) mcx_transport(const KArgs a) {
 
     Photon s;
     unsigned int vt = 0;
-    bool claimed = claim_vt(a, ps, vt);
+    bool claimed = (threadIdx.x & 31u) < a.lanes && claim_vt(a, ps, vt);
     bool relaunch = false;         /* a relaunch request from the previous step */
     unsigned int relaunch_isdet = 0;
     bool fresh = true;             /* vt just claimed: initial launch */

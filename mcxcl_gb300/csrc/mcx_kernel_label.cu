@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(LB_BLOCK, 4) mcx_transport_label(const KArgs a
        detector bit */
     bool offgrid = false;
     s.f.x = 1.f;
-    int st = lb_claim(a, vt);
+    int st = (threadIdx.x & 31u) < a.lanes ? lb_claim(a, vt) : DONE;
 
     while (__any_sync(0xFFFFFFFFu, st != DONE)) {
         if (st == ENDED || st == FRESH) {

@@ -32,6 +32,7 @@ struct KArgs {
     float2* detw;                  /* maxdetphoton x {weight, time of flight} when detected, or null */
     unsigned int* detcount;
     unsigned int* vtcounter;       /* work queue head */
+    unsigned int lanes;            /* lanes of each warp that take work (32 but for small runs) */
     unsigned int* status;
     unsigned long long* counters;  /* step, scatter, launch, reflect, failed */
     /* replay: per photon, the saved RNG state, detected weight, time of flight, detector id */
