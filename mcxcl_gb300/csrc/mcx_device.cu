@@ -506,15 +506,39 @@ void shape_for(unsigned long long photons, int sms, bool label, int* blocks, uns
     }
 }
 
-/* the configurations of mcx_transport_label beyond what the common
-   instantiations fix: one byte a voxel, one source, launched photons that
-   deposit flux, fluence or energy, no scattering count at which g drops to 0
-   (a float count of scatterings stops below 2^24 + 1), 15-bit voxel indices */
-bool label_config(const mcxg_kparams& kp) {
-    return kp.mediaword == 1 && !kp.replay && kp.save2pt && !kp.extrasrclen && kp.gscatter > (1u << 24) &&
-           (kp.outputtype == otFlux || kp.outputtype == otFluence || kp.outputtype == otEnergy ||
-            kp.outputtype >= otAdjoint) &&
-           kp.dimx < 32768u && kp.dimy < 32768u && kp.dimz < 32768u;
+/* What mcx_transport_label does for a run (RUN_FWD ..), or -1: it takes 3-D
+   volumes of byte labels or float absorption with one Henyey-Greenstein source
+   and no scattering count at which g drops to 0 (a float count of scatterings
+   stops below 2^24 + 1), voxel indices of 15 bits; deposits of flux, fluence
+   or energy, the replays that deposit path or scatterings, modulated sources
+   in label volumes, and the passes of the fluence gradient */
+int label_run(const mcxg_kparams& kp, unsigned int adjmode) {
+    const bool labels = kp.mediaword == 1 && kp.mediaformat <= 4;
+    const bool mua = kp.mediaformat == 101 && kp.mediaword == 4 && kp.medianum >= 2;
+    if (!(labels || mua) || kp.is2d || kp.nphase > 2 || kp.srcnum > 1 || !kp.save2pt || kp.extrasrclen ||
+            kp.gscatter <= (1u << 24) || kp.dimx > 32767u || kp.dimy > 32767u || kp.dimz > 32767u) {
+        return -1;
+    }
+    if (adjmode) {
+        return adjmode == 1u ? mcxg::RUN_ADJ1 : mcxg::RUN_ADJ2;
+    }
+    if (kp.omega > 0.f && !kp.replay) {
+        return labels ? mcxg::RUN_RF : -1;
+    }
+    switch (kp.outputtype) {
+    case otJacobian:
+    case otWLTOF:
+        return kp.replay ? mcxg::RUN_JAC : -1;
+    case otWP:
+    case otDCS:
+    case otWPTOF:
+        return kp.replay ? mcxg::RUN_SITE : -1;
+    case otL:
+    case otRF:
+    case otRFmus:
+        return -1;
+    }
+    return mcxg::RUN_FWD;
 }
 
 /* its shared memory: 32 B of launch-time state a thread, three property rows
@@ -1449,11 +1473,13 @@ int mcxg_simulate(mcxg_session* s, unsigned int flags, float* kernel_ms) {
             s->tile_used = t;
         }
     }
-    /* byte-label volumes in the usual configuration have a kernel of their own */
-    const bool label = !exact && common && label_config(kp) && block == mcxg::kLabelBlock &&
-                       !(lflags & (mcxg::LF_WAGG | mcxg::LF_TILE | mcxg::LF_ACC64 | mcxg::LF_ADJ));
+    /* the usual configurations have a kernel of their own */
+    const int lrun = (exact || pol || svmc || xmedia || s->maxjump || (flags & MCXG_GENERAL) || block != mcxg::kLabelBlock ||
+                      (lflags & (mcxg::LF_WAGG | mcxg::LF_TILE | mcxg::LF_ACC64))) ? -1 : label_run(kp, adjmode);
+    const bool label = lrun >= 0;
     if (label) {
-        lflags |= (int)(kp.savedetflag & 0xEu) << mcxg::LF_KINDS;
+        lflags |= (kp.mediaformat == 101 ? mcxg::LF_MUA : 0) | lrun << mcxg::LF_RUN |
+                  (int)(kp.savedetflag & 0xEu) << mcxg::LF_KINDS;
         smem = label_shared_bytes(kp);
     }
     if (label && !s->up_label) {
@@ -1469,7 +1495,7 @@ int mcxg_simulate(mcxg_session* s, unsigned int flags, float* kernel_ms) {
     }
     int bpsm = exact ? 2 : bpsm_sel;
     a.lanes = 32;
-    if (!exact && !adjmode && !s->block_req && !s->bpsm_req) {
+    if (!exact && adjmode != 2u && !s->block_req && !s->bpsm_req) {
         int few = 0;
         shape_for((unsigned long long)kp.threadphoton * kp.nthread + (unsigned long long)std::max(kp.oddphoton, 0),
                   s->info.sm, label, &few, &a.lanes);

@@ -89,7 +89,9 @@ struct KArgs {
 /* flag bits for the launch entries */
 enum { LF_DET = 1, LF_REFL = 2, LF_WAGG = 4, LF_CAPPED = 8, LF_XMEDIA = 32, LF_COMMON = 64, LF_RF = 128, LF_POL = 256, LF_SVMC = 512,
        LF_ACC64 = 1024, LF_ADJ = 2048, LF_TILE = 4096,
-       LF_KINDS = 16 /* bit position of savedetflag's partial-data bits, for the label kernel */ };
+       /* for the label kernel: float absorption; bit positions of what the run
+          does (RUN_FWD .. RUN_ADJ2) and of savedetflag's partial-data bits */
+       LF_MUA = 8192, LF_RUN = 16, LF_KINDS = 20 };
 
 /* fast instantiation: hardware transcendental approximations */
 cudaError_t fast_upload(const mcxg_kparams* p, const float* det4, unsigned int ndet, const float* srcx16,
@@ -97,6 +99,16 @@ cudaError_t fast_upload(const mcxg_kparams* p, const float* det4, unsigned int n
 cudaError_t fast_launch(const KArgs& a, int flags, int grid, int block, size_t smem, cudaStream_t st);
 cudaError_t fast_occupancy(int flags, int block, size_t smem, int* blocks_per_sm);
 cudaError_t fast_attributes(int flags, cudaFuncAttributes* attr);
+
+/* what a run of the label kernel does */
+enum {
+    RUN_FWD,    /* deposits flux, fluence or energy */
+    RUN_JAC,    /* replay: the detected weight (x time of flight) times the path in each voxel */
+    RUN_SITE,   /* replay: the detected weight (x time of flight, x 1 - cos theta) at each scattering */
+    RUN_RF,     /* modulated source: complex weight and field */
+    RUN_ADJ1,   /* fluence gradient: each photon's loss total */
+    RUN_ADJ2    /* ... and the gradients */
+};
 
 constexpr int kLabelBlock = 256;   /* its threads a block */
 /* the kernel of byte-label volumes in the usual configuration (one source: no extra-source table) */

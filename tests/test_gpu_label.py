@@ -1,4 +1,4 @@
-"""The kernel of byte-label volumes against the general common-configuration one.
+"""The kernel of the usual configurations (byte labels or float absorption) against the general one.
 
 Both run the same photons with the same arithmetic, so every output is compared to the last bit where it is
 summed exactly (energies, records, launch states) and to the rounding of the float remainders in the field:
@@ -25,6 +25,10 @@ def _void_inside():
 
 _ODD = dict(vol=_void_inside(), srcpos=[18, 14, 0], detpos=[[18, 6, 0, 2], [30, 14, 0, 3]],
             prop=[[0, 0, 1, 1], [0.01, 1, 0.5, 1.37], [0.02, 5, 0.9, 1.45], [0.3, 12, 0.0, 1.37]])
+_MAP = (0.005 + 0.02 * np.random.RandomState(3).rand(37, 29, 41)).astype(np.float32)
+_MAP[13:17, 12:18, 18:24] = 0
+_MAP[30:, :, 20:] = 1e-8
+_MUA = dict(vol=_MAP[None], srcpos=[18, 14, 0], detpos=[[18, 6, 0, 2], [30, 14, 0, 3]], prop=[[0, 0, 1, 1], [0.01, 1, 0.77, 1.37]])
 CASES = {
     "default": {}, "plain": dict(issavedet=0, issaveseed=0), "paths": dict(savedetflag="dp"), "scatterings": dict(savedetflag="ds"),
     "both": dict(savedetflag="dsp"), "momentum": dict(savedetflag="dspm"), "id": dict(savedetflag="d"),
@@ -38,14 +42,22 @@ CASES = {
     "one voxel": cases.VARIANTS["onevoxel"], "few photons": dict(nphoton=100), "specular": cases.VARIANTS["outside_src_specular"],
     "wide label": dict(vol=np.full((40, 40, 40), 127, np.uint8), prop=[[0, 0, 1, 1]] + [[0.01, 1, 0.5, 1.37]] * 127, savedetflag="d"),
     "angles": cases.VARIANTS["angleinvcdf"], "pattern": cases.VARIANTS["pattern"], "isotropic": cases.VARIANTS["isotropic"],
-    "many gates": dict(tstep=2e-11), "no photon detected": dict(detpos=[[20, 20, 39, 1]], nphoton=50),
+    "many gates": dict(tstep=2e-11), "backward": dict(prop=[[0, 0, 1, 1], [0.01, 2, -0.4, 1.37], [0.02, 5, 0.87, 1.45]]),
+    # float absorption: voxels without any, and every record kind
+    "mua": dict(_MUA, savedetflag="dxv"), "mua energy": dict(_MUA, outputtype="energy"), "mua plain": dict(_MUA, issavedet=0, issaveseed=0),
+    "mua matched": dict(_MUA, isreflect=0, savedetflag="dspm", minenergy=0.01), "mua gates": dict(_MUA, tstart=1e-10, tend=1.7e-9, tstep=1e-10),
+    "mua mirror": dict(_MUA, bc="mmammm"), "mua cyclic": dict(_MUA, bc="ccrrcc", isreflect=0),
+    # modulated sources
+    "rf": dict(omega=2 * np.pi * 1e8), "rf roulette": dict(omega=2 * np.pi * 3e8, minenergy=0.01, outputtype="fluence"),
+    "rf odd": dict(_ODD, omega=2 * np.pi * 1e8, isreflect=0, issavedet=0, issaveseed=0),
+    "rf no absorption": dict(omega=2 * np.pi * 1e8, prop=[[0, 0, 1, 1], [0, 1, 0.5, 1.37], [1e-8, 5, 0.9, 1.45]]), "no photon detected": dict(detpos=[[20, 20, 39, 1]], nphoton=50),
 }
 
 
 def _run(cfg, general):
     import mcxcl_gb300
     r = mcxcl_gb300.run(dict(cfg, **({"gscatter": 1 << 24} if general else {})))
-    out = {"flux": np.asarray(r["flux"], np.float64)}
+    out = {"flux": np.asarray(r["flux"], np.complex128 if np.iscomplexobj(r["flux"]) else np.float64)}
     for k in ("energytot", "energyabs", "detected", "failedlaunch"):
         out[k] = r["stat"][k]
     if "dref" in r:
@@ -68,3 +80,44 @@ def test_same_photons_as_the_general_kernel(name):
         if k in a:
             assert np.linalg.norm(a[k] - b[k]) <= 1e-6 * np.linalg.norm(b[k]), k
             assert np.array_equal(a[k] != 0, b[k] != 0), k
+
+
+@pytest.mark.parametrize("base", ["default", "odd", "mua", "roulette"])
+@pytest.mark.parametrize("output", ["jacobian", "wltof", "nscat", "wm", "wptof", "flux", "energy"])
+@pytest.mark.parametrize("det", [-1, 0, 2])
+def test_replays_as_the_general_kernel(base, output, det):
+    """A replay's deposits: weight x path or x scatterings, per detector and gate."""
+    import mcxcl_gb300
+    cfg = cases.small_two_media(**dict(dict(nphoton=50000, savedetflag="dsp", tstep=5e-10), **CASES[base]))
+    if base == "mua":
+        cfg["savedetweight"] = 1
+    first = mcxcl_gb300.run(cfg)
+    rep = dict(cfg, seed=first["seeds"], outputtype=output, replaydet=det, savedetflag="dsp")
+    if base == "mua":
+        rep.update(replayweight=first["detweight"][0], replaytof=first["detweight"][1].clip(0, 4.99e-9),
+                   replaydetid=first["detp"][0].astype(np.int32))
+    else:
+        rep["detphotons"] = first["detp"]
+    a, b = _run(rep, False), _run(rep, True)
+    assert a["energytot"] == b["energytot"] and a["energyabs"] == b["energyabs"] and a["detected"] == b["detected"]
+    assert np.linalg.norm(b["flux"]) > 0 and np.linalg.norm(a["flux"] - b["flux"]) <= 1e-6 * np.linalg.norm(b["flux"])
+
+
+@pytest.mark.parametrize("name", ["default", "odd", "mua", "no absorption", "mua gates"])
+def test_fluence_gradient_as_the_general_kernel(name):
+    """The loss gradient's float sums add the same terms in another order: up to 1e5 terms of one sign in an
+    element, each sum off by at most a few hundred roundings of 6e-8."""
+    from mcxcl_gb300 import diff
+    cfg = cases.small_two_media(**dict(dict(nphoton=50000), **CASES[name]))
+    for k in ("issaveseed", "savedetflag"):
+        cfg.pop(k, None)
+    cfg["issavedet"] = 0
+    got = []
+    for extra in ({}, {"gscatter": 1 << 24}):
+        g = diff.FluenceGradient(dict(cfg, **extra))
+        f = g.forward()
+        d = np.random.RandomState(1).standard_normal(f.shape)
+        got.append((f, *g.backward(d)))
+        g.close()
+    for x, y in zip(*got):
+        assert np.linalg.norm(y) > 0 and np.linalg.norm(x - y) <= 2e-5 * np.linalg.norm(y)
