@@ -30,7 +30,7 @@ UNITS = {
     "mcx_kernel_exact.cu": ["-fmad=false", "-prec-div=true", "-prec-sqrt=true", "-ftz=false"],
     "mcx_device.cu": [],
 }
-HEADERS = ["mcx_kernel.cuh", "mcx_pmath.cuh", "mcx_kparams.h", "mcx_launch.h"]
+HEADERS = ["mcx_kernel.cuh", "mcx_kernel_label.cuh", "mcx_pmath.cuh", "mcx_kparams.h", "mcx_launch.h"]
 
 
 def _nvcc():

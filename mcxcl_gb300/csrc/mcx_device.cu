@@ -2058,7 +2058,7 @@ int batch_enqueue(mcxg_session* s, int lflags) {
         MCXG_TRY(cudaMemsetAsync(s->d_words + 1, 0, sizeof(unsigned int), s->st));
         a.simctr = s->d_simctr + w0;
         a.nsim = n;
-        MCXG_TRY(mcxg::batch_launch(a, lflags, s->bt_grid, s->bt_block, (size_t)s->bt_block * 32, s->st));
+        MCXG_TRY(mcxg::batch_launch(a, lflags, s->bt_grid, s->bt_block, s->st));
     }
     batch_energy<<<s->nsim, 256, 0, s->st>>>(s->d_benergy, s->d_sims, s->d_bsum);
     return MCXG_OK;
@@ -2170,10 +2170,11 @@ int mcxg_batch_simulate(mcxg_session* s, unsigned int flags, float* kernel_ms) {
         return MCXG_ERR_STATE;
     }
     MCXG_TRY(cudaSetDevice(s->device));
-    bool refl = false, common = true;
+    bool refl = false, common = true, label = true;
     for (const mcxg_simdesc& d : s->h_sims) {
         refl = refl || d.kp.dorefl_compiled;
         common = common && !d.kp.is2d && d.kp.mediaformat <= 4 && d.kp.nphase <= 2;
+        label = label && label_run(d.kp, 0u) == mcxg::RUN_FWD;
     }
     const bool verify = (flags & MCXG_VERIFY) != 0;
     if (verify) {
@@ -2201,8 +2202,11 @@ int mcxg_batch_simulate(mcxg_session* s, unsigned int flags, float* kernel_ms) {
     int lflags = (refl ? mcxg::LF_REFL : 0) | (agg ? mcxg::LF_WAGG : 0) | (bpsm_req >= 3 ? mcxg::LF_CAPPED : 0) |
                  (common && !(flags & MCXG_GENERAL) ? mcxg::LF_COMMON : 0) | (verify ? mcxg::LF_ACC64 : 0);
     const int block = s->block_req ? s->block_req : 256;
+    if (label && !agg && !verify && !(flags & MCXG_GENERAL) && block == mcxg::kLabelBlock) {
+        lflags |= mcxg::LF_LABEL;
+    }
     int occ = 0;
-    MCXG_TRY(mcxg::batch_occupancy(lflags, block, (size_t)block * 32, &occ));
+    MCXG_TRY(mcxg::batch_occupancy(lflags, block, std::min<uint32_t>(s->nsim, mcxg::kBatchWave), &occ));
     int bpsm = std::max(1, std::min(bpsm_req, occ > 0 ? occ : bpsm_req));
     const int grid = s->info.sm * bpsm;
     if (grid != s->bt_grid || block != s->bt_block) {

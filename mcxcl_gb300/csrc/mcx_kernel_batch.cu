@@ -7,6 +7,7 @@
  */
 #define MCXG_BATCH_TU
 #include "mcx_kernel.cuh"
+#include "mcx_kernel_label.cuh"
 #include "mcx_launch.h"
 
 namespace mcxg {
@@ -46,6 +47,10 @@ static void* kbatch_acc64() {
 
 static void* select(int flags) {
     const bool refl = flags & LF_REFL, wagg = flags & LF_WAGG, cap = flags & LF_CAPPED;
+    if (flags & LF_LABEL) {
+        return refl ? (void*)mcx_transport_label<RUN_FWD, VOL_LABEL, DET_NONE, true>
+                    : (void*)mcx_transport_label<RUN_FWD, VOL_LABEL, DET_NONE, false>;
+    }
     if (flags & LF_ACC64) {
         return (flags & LF_COMMON) ? (refl ? kbatch_acc64<true, true>() : kbatch_acc64<false, true>())
                                    : (refl ? kbatch_acc64<true, false>() : kbatch_acc64<false, false>());
@@ -53,12 +58,25 @@ static void* select(int flags) {
     return (flags & LF_COMMON) ? kshape<true>(refl, wagg, cap) : kshape<false>(refl, wagg, cap);
 }
 
-cudaError_t batch_launch(const KArgs& a, int flags, int grid, int block, size_t smem, cudaStream_t st) {
-    void* args[] = {(void*)&a};
-    return cudaLaunchKernel(select(flags), dim3(grid), dim3(block), args, smem, st);
+size_t batch_shared_bytes(int flags, int block, unsigned int nsim) {
+    return (size_t)block * sizeof(ColdState) +
+           ((flags & LF_LABEL) ? (size_t)nsim * LabelPS<VOL_LABEL, DET_NONE>::kSim * sizeof(float4) : 0);
 }
 
-cudaError_t batch_occupancy(int flags, int block, size_t smem, int* blocks_per_sm) {
+cudaError_t batch_launch(const KArgs& a, int flags, int grid, int block, cudaStream_t st) {
+    void* args[] = {(void*)&a};
+    return cudaLaunchKernel(select(flags), dim3(grid), dim3(block), args, batch_shared_bytes(flags, block, a.nsim), st);
+}
+
+/* resident blocks a SM; also admits the shared memory of a wave of nsim */
+cudaError_t batch_occupancy(int flags, int block, unsigned int nsim, int* blocks_per_sm) {
+    const size_t smem = batch_shared_bytes(flags, block, nsim);
+    if (smem > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(select(flags), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) {
+            return e;
+        }
+    }
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, select(flags), block, smem);
 }
 

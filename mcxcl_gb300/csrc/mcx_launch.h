@@ -91,7 +91,8 @@ enum { LF_DET = 1, LF_REFL = 2, LF_WAGG = 4, LF_CAPPED = 8, LF_XMEDIA = 32, LF_C
        LF_ACC64 = 1024, LF_ADJ = 2048, LF_TILE = 4096,
        /* for the label kernel: float absorption; bit positions of what the run
           does (RUN_FWD .. RUN_ADJ2) and of savedetflag's partial-data bits */
-       LF_MUA = 8192, LF_RUN = 16, LF_KINDS = 20 };
+       LF_MUA = 8192, LF_RUN = 16, LF_KINDS = 20,
+       LF_LABEL = 1 << 24 /* batches: that kernel */ };
 
 /* fast instantiation: hardware transcendental approximations */
 cudaError_t fast_upload(const mcxg_kparams* p, const float* det4, unsigned int ndet, const float* srcx16,
@@ -127,8 +128,8 @@ cudaError_t exact_rngdump(const KArgs& a, int grid, int block, cudaStream_t st);
    memory (from device memory), then the launch */
 constexpr int kBatchWave = 136;
 cudaError_t batch_wave_upload(const mcxg_simdesc* d_descs, unsigned int n, cudaStream_t st);
-cudaError_t batch_launch(const KArgs& a, int flags, int grid, int block, size_t smem, cudaStream_t st);
-cudaError_t batch_occupancy(int flags, int block, size_t smem, int* blocks_per_sm);
+cudaError_t batch_launch(const KArgs& a, int flags, int grid, int block, cudaStream_t st);
+cudaError_t batch_occupancy(int flags, int block, unsigned int nsim, int* blocks_per_sm);
 }  // namespace mcxg
 
 #endif

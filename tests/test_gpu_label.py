@@ -121,3 +121,28 @@ def test_fluence_gradient_as_the_general_kernel(name):
         g.close()
     for x, y in zip(*got):
         assert np.linalg.norm(y) > 0 and np.linalg.norm(x - y) <= 2e-5 * np.linalg.norm(y)
+
+
+def _batch():
+    """150 simulations (two waves) of different volumes, media, gates and outputs, in 1 to 3 photons a thread."""
+    sims = []
+    for k in range(150):
+        name = ["default", "noreflect", "energy", "fluence", "cyclic", "mirror", "roulette", "unit", "matched", "no absorption", "odd gates",
+                "isotropic", "few photons", "backward"][k % 14]
+        cfg = cases.small_two_media(**dict(dict(nphoton=1500), **CASES[name]))
+        for key in ("detpos", "savedetflag", "issaveseed"):
+            cfg.pop(key, None)
+        sims.append(dict(cfg, seed=k + 1, issavedet=0))
+    return sims
+
+
+@pytest.mark.parametrize("per_thread", [0, 3])
+def test_batch_as_the_general_kernel(per_thread):
+    import mcxcl_gb300
+    sims = _batch()
+    a = mcxcl_gb300.run_batch(sims, photons_per_thread=per_thread)
+    b = mcxcl_gb300.run_batch([dict(c, gscatter=1 << 24) for c in sims], photons_per_thread=per_thread)
+    for x, y in zip(a, b):
+        assert x["stat"]["energytot"] == y["stat"]["energytot"] and x["stat"]["energyabs"] == y["stat"]["energyabs"]
+        f, g = np.asarray(x["flux"], np.float64), np.asarray(y["flux"], np.float64)
+        assert np.linalg.norm(g) > 0 and np.linalg.norm(f - g) <= 1e-6 * np.linalg.norm(g)
