@@ -511,7 +511,7 @@ void shape_for(unsigned long long photons, int sms, bool label, int* blocks, uns
    and no scattering count at which g drops to 0 (a float count of scatterings
    stops below 2^24 + 1), voxel indices of 15 bits; deposits of flux, fluence
    or energy, the replays that deposit path or scatterings, modulated sources
-   in label volumes, and the passes of the fluence gradient */
+   in label volumes, and the first pass of the fluence gradient */
 int label_run(const mcxg_kparams& kp, unsigned int adjmode) {
     const bool labels = kp.mediaword == 1 && kp.mediaformat <= 4;
     const bool mua = kp.mediaformat == 101 && kp.mediaword == 4 && kp.medianum >= 2;
@@ -520,7 +520,9 @@ int label_run(const mcxg_kparams& kp, unsigned int adjmode) {
         return -1;
     }
     if (adjmode) {
-        return adjmode == 1u ? mcxg::RUN_ADJ1 : mcxg::RUN_ADJ2;
+        /* the second pass stays where it was: its float sums drop up to 1e-4 of the
+           hottest voxels' gradients, how much depends on the order of the additions */
+        return adjmode == 1u ? mcxg::RUN_ADJ1 : -1;
     }
     if (kp.omega > 0.f && !kp.replay) {
         return labels ? mcxg::RUN_RF : -1;

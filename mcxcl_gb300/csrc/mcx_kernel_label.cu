@@ -46,8 +46,6 @@ static void* kvol(int flags) {
         return kany<RUN_SITE, VOL>(flags);
     case RUN_ADJ1:
         return krefl<RUN_ADJ1, VOL, DET_NONE>(flags);
-    case RUN_ADJ2:
-        return krefl<RUN_ADJ2, VOL, DET_NONE>(flags);
     }
     if (!(flags & LF_DET)) {
         return krefl<RUN_FWD, VOL, DET_NONE>(flags);

@@ -3,7 +3,7 @@
  *
  * Byte labels or float absorption, three dimensions, Henyey-Greenstein, one
  * source; deposits of flux, fluence or energy, replays, modulated sources
- * and the passes of the fluence gradient -- each with all of that fixed at
+ * and the first pass of the fluence gradient -- each with all of that fixed at
  * compile time.  The photons, their random numbers and every
  * rounding are those of mcx_transport (mcx_kernel.cuh), whose device
  * functions it shares; what differs is what a step costs.
@@ -22,7 +22,7 @@
  * 1e6 photons 8.95 -> 6.0 ms; cube + sphere with detectors, 1e6 14.1 -> 8.9 ms, 2e7
  * 113 -> 79 ms; head, 1e7 42.9 -> 32 ms.  Calls: modulated sphere 1e6 18.0 -> 10.2 ms,
  * replay of 9,000 photons 4.9 -> 3.1 ms, readings and their gradient on a
- * 100^3 absorption map 23.5 -> 14.6 ms, fluence gradient 47 -> 36 ms.
+ * 100^3 absorption map 23.5 -> 14.6 ms, fluence gradient 47 -> 39 ms.
  */
 #ifndef MCX_KERNEL_LABEL_CUH
 #define MCX_KERNEL_LABEL_CUH
@@ -374,8 +374,8 @@ template <int KIND, int VOL, int DET, bool REFL>
 __global__ void __launch_bounds__(LB_BLOCK, KIND == RUN_RF ? 3 : 4) mcx_transport_label(const KArgs a) {
     typedef Mth<false> M;
     typedef Voxel<VOL> V;
-    constexpr bool GEN = VOL == VOL_MUA || KIND == RUN_RF || KIND == RUN_ADJ1 || KIND == RUN_ADJ2;
-    constexpr bool JAC = KIND == RUN_JAC, SITE = KIND == RUN_SITE, RF = KIND == RUN_RF, ADJ = KIND == RUN_ADJ1 || KIND == RUN_ADJ2;
+    constexpr bool GEN = VOL == VOL_MUA || KIND == RUN_RF || KIND == RUN_ADJ1;
+    constexpr bool JAC = KIND == RUN_JAC, SITE = KIND == RUN_SITE, RF = KIND == RUN_RF, ADJ = KIND == RUN_ADJ1;
     typedef LabelPS<VOL, DET> PS;
     PS ps;
     Shared S;
@@ -395,14 +395,14 @@ __global__ void __launch_bounds__(LB_BLOCK, KIND == RUN_RF ? 3 : 4) mcx_transpor
     bool offgrid = false;
     s.f.x = 1.f;
     Replayed rp = {0.f, 1.f, 0u};
-    float adjJ = 0.f, adjP = 0.f;          /* fluence gradient: the photon's loss total and its running part */
+    float adjJ = 0.f;                      /* fluence gradient: the photon's loss total */
     int st = (threadIdx.x & 31u) < a.lanes ? ps.claim(a, vt) : DONE;
 
     while (__any_sync(0xFFFFFFFFu, st != DONE)) {
         if (st == ENDED || st == FRESH) {
             const mcxg_kparams& c_p = ps.p();
             bool go = true;
-            if (KIND == RUN_ADJ1 && st == ENDED) {
+            if (ADJ && st == ENDED) {
                 a.adjJ[adj_slot(c_p, vt, s.f.w)] = adjJ;
             }
             if (st == ENDED && closephoton<DET != DET_NONE, false, false>(a, ps, S, s, endflag, vt)) {
@@ -434,10 +434,7 @@ __global__ void __launch_bounds__(LB_BLOCK, KIND == RUN_RF ? 3 : 4) mcx_transpor
                     if (JAC || SITE) {
                         rp = replayed<KIND>(a, ps, vt, s.f.w);
                     }
-                    if (ADJ) {
-                        adjP = 0.f;
-                        adjJ = KIND == RUN_ADJ2 ? a.adjJ[adj_slot(c_p, vt, s.f.w)] : 0.f;
-                    }
+                    adjJ = 0.f;
                     cx = (float)s.fx + 0.5f;
                     cy = (float)s.fy + 0.5f;
                     cz = (float)s.fz + 0.5f;
@@ -473,10 +470,6 @@ __global__ void __launch_bounds__(LB_BLOCK, KIND == RUN_RF ? 3 : 4) mcx_transpor
                         1.f - ctheta;
                 }
                 rotate_rn<GEN>(s.v, stheta, ctheta, sphi, cphi);
-                if (KIND == RUN_ADJ2) {
-                    /* a scattering in this voxel: 1/mus on every later deposit */
-                    atomicAdd(a.field + c_p.fieldlen + s.idx1d, (adjJ - adjP) * ps.row(label, 0).w);
-                }
                 if (SITE) {
                     const unsigned int key = s.idx1d + rp.off;
                     if (rp.off != Replayed::kBad && key < c_p.fieldlen) {
@@ -588,20 +581,7 @@ __global__ void __launch_bounds__(LB_BLOCK, KIND == RUN_RF ? 3 : 4) mcx_transpor
                             const bool dep = inwin & (fabsf(weight) > 0.f);
                             /* the visit that just ended, in voxel idxold */
                             const float c = dep ? __ldg(a.adjc + key) : 0.f;
-                            const float cD = c * weight;
-                            if (KIND == RUN_ADJ1) {
-                                adjJ += cD;
-                            } else {
-                                const float l = s.pathlen, rest = adjJ - adjP;
-                                float own = 0.f;
-                                if (dep) {
-                                    own = (A.x < K_EPS) ? -0.5f * c * s.w0 * l * l
-                                                        : c * (s.p.w * l - weight) * __fdividef(1.f, A.x);
-                                }
-                                atomicAdd(a.field + idxold, own - l * (rest - cD));
-                                atomicAdd(a.field + c_p.fieldlen + idxold, -l * rest);
-                                adjP += cD;
-                            }
+                            adjJ = __fadd_rn(adjJ, __fmul_rn(c, weight));
                         }
                     } else if (left & (s.f.y >= h1.z) & (s.f.y < h1.x) & (fabsf(weight) > 0.f)) {
                         /* field_split and field_commit: the rounded product is a float
