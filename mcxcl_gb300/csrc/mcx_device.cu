@@ -500,7 +500,7 @@ void shape_for(unsigned long long photons, int sms, bool label, int* blocks, uns
         *lanes = std::max(1u, (unsigned int)(q + 15) / 16);       /* one photon a lane, over 16 warps */
     } else if (q <= 1000) {
         *blocks = 1;
-        *lanes = std::min(32u, (unsigned int)(q + 11) / 12);
+        *lanes = std::min(32u, (unsigned int)(q + 7) / 8);
     } else {
         *blocks = !label ? 4 : (q <= 10000 ? 2 : (q <= 35000 ? 3 : 4));
     }

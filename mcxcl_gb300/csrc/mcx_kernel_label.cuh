@@ -507,11 +507,12 @@ __global__ void __launch_bounds__(LB_BLOCK, KIND == RUN_RF ? 3 : 4) mcx_transpor
                 M::sincos(__fmul_rn(K_TWO_PI, __fsub_rn(rnd12(s.t), 1.f)), &sphi, &cphi);
                 const float u = __fsub_rn(rnd12(s.t), 1.f);
                 const float4 g = ps.row(label, 1);
-                float ctheta = 2.f * u - 1.f;
-                if (fabsf(g.z) > 2.f * K_EPS) {
+                float ctheta;
+                {
                     const float t = __fmul_rn(g.x, rcp_approx(__fmaf_rn(g.z, u, g.y)));
                     const float d = GEN ? __fsub_rn(g.w, __fmul_rn(t, t)) : __fmaf_rn(-t, t, g.w);
                     ctheta = fmaxf(-1.f, fminf(1.f, __fmul_rn(d, ps.row(label, 2).x)));
+                    ctheta = fabsf(g.z) > 2.f * K_EPS ? ctheta : 2.f * u - 1.f;
                 }
                 const float stheta = M::sqrt(__fmaf_rn(-ctheta, ctheta, 1.f));
                 if (DET == DET_SP || (DET == DET_ANY && SAVE_NSCAT(c_p.savedetflag) && recorded)) {
@@ -650,9 +651,7 @@ __global__ void __launch_bounds__(LB_BLOCK, KIND == RUN_RF ? 3 : 4) mcx_transpor
                         if (PS::kBatch) {
                             key += __float_as_uint(ps.hot(4).z);
                         }
-                        if (kf != 0.f) {
-                            atomicAdd(a.fhi + key, (unsigned long long)__float2ll_rn(kf));
-                        }
+                        atomicAdd(a.fhi + key, (unsigned long long)__float2ll_rn(kf));
                         if (r != 0.f) {
                             atomicAdd(a.flo + key, r);
                         }
