@@ -56,6 +56,9 @@ struct mcxg_session {
     float* d_traj = nullptr;
     size_t traj_cap = 0, jump_cap = 0;
     uint32_t maxjump = 0;
+    uint32_t* d_lfpow = nullptr;     /* powers of the generator's step for blocks of lfpow_len words */
+    size_t lfpow_cap = 0;
+    uint32_t lfpow_len = 0, lfpow_n = 0;
     uint32_t* d_lfib = nullptr;      /* 31-word generator windows, one per block of seed words */
     size_t lfib_cap = 0;
     float* d_field = nullptr;        /* per component: hi, lo, spill count planes (3 x fieldlen) */
@@ -217,16 +220,28 @@ __global__ void energy_partials(const float2* __restrict__ e, unsigned int n, do
     }
 }
 
-/* fixed-order final sum, so the result is the same bits on every run */
-__global__ void energy_final(double* part, int nblocks) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        double a = 0.0, b = 0.0;
-        for (int i = 0; i < nblocks; i++) {
-            a += part[i * 2];
-            b += part[i * 2 + 1];
+/* final sum in an order fixed by the number of blocks, so the result is the
+   same bits on every run; one block: a serial loop over 608 partials took 30 us,
+   a tree 4 */
+__global__ void __launch_bounds__(256) energy_final(double* part, int nblocks) {
+    double a = 0.0, b = 0.0;
+    for (int i = threadIdx.x; i < nblocks; i += 256) {
+        a += part[i * 2];
+        b += part[i * 2 + 1];
+    }
+    __shared__ double wa[256], wb[256];
+    wa[threadIdx.x] = a;
+    wb[threadIdx.x] = b;
+    for (int o = 128; o > 0; o >>= 1) {
+        __syncthreads();
+        if ((int)threadIdx.x < o) {
+            wa[threadIdx.x] += wa[threadIdx.x + o];
+            wb[threadIdx.x] += wb[threadIdx.x + o];
         }
-        part[nblocks * 2] = a;
-        part[nblocks * 2 + 1] = b;
+    }
+    if (threadIdx.x == 0) {
+        part[nblocks * 2] = wa[0];
+        part[nblocks * 2 + 1] = wb[0];
     }
 }
 
@@ -247,12 +262,47 @@ __device__ __forceinline__ double merged_at(const float* __restrict__ f, size_t 
     return cell_value(f, total, unit, i);
 }
 
-__global__ void field_merge_f32(const float* __restrict__ f, size_t n, size_t total, double unit, double scale,
-                                float* __restrict__ out) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        size_t j;
-        out[i] = (float)(merged_at(f, n, total, unit, i, j) * scale);
+/* (count x unit + remainder) x scale rounded to float, the same bits as
+   cell_value() * scale, with the FP64 pipe (two operations a cycle and SM)
+   left to what needs it: nothing for an untouched element, and without a
+   remainder one product, unit being a power of two. */
+__device__ __forceinline__ float merged_f32(long long k, float r, double unit, double scale) {
+    if (r != 0.f) {
+        return (float)(((double)k * unit + (double)r) * scale);
     }
+    return k ? (float)((double)k * (unit * scale)) : 0.f;
+}
+
+/* out[i] = merged_f32() of the elements [0, n) from `first` on, scaled by
+   scale(i): four elements' loads in flight a thread */
+template <class Scale>
+__device__ __forceinline__ void merge_range(const float* __restrict__ f, size_t total, size_t first, size_t n, double unit,
+                                            Scale scale, float* __restrict__ out) {
+    const long long* hi = reinterpret_cast<const long long*>(f) + first;
+    const float* lo = f + 2 * total + first;
+    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += 4 * stride) {
+        long long k[4];
+        float r[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const size_t j = i + u * stride;
+            k[u] = j < n ? __ldcs(hi + j) : 0ll;
+            r[u] = j < n ? __ldcs(lo + j) : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const size_t j = i + u * stride;
+            if (j < n) {
+                out[first + j] = (k[u] | (long long)__float_as_uint(r[u])) ? merged_f32(k[u], r[u], unit, scale(j)) : 0.f;
+            }
+        }
+    }
+}
+
+__global__ void field_merge_f32(const float* __restrict__ f, size_t total, double unit, double scale,
+                                float* __restrict__ out) {
+    merge_range(f, total, 0, total, unit, [=](size_t) { return scale; }, out);
 }
 
 /* element j belongs to source j % nsrc (photon sharing interleaves the
@@ -268,11 +318,7 @@ __global__ void field_merge_interleaved(const float* __restrict__ f, size_t n, s
 
 __global__ void field_merge_blocks(const float* __restrict__ f, size_t n, size_t total, double unit, size_t blocklen,
                                    const double* __restrict__ scales, float* __restrict__ out) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        size_t j;
-        const double v = merged_at(f, n, total, unit, i, j);
-        out[i] = (float)(v * scales[j / blocklen]);
-    }
+    merge_range(f, total, 0, total, unit, [=](size_t i) { return scales[(i % n) / blocklen]; }, out);
 }
 
 /* reciprocals of each simulation's property rows, as the single-simulation
@@ -290,14 +336,20 @@ __global__ void batch_recip(mcxg_simdesc* __restrict__ sims, unsigned int nsim) 
     }
 }
 
-/* per-simulation FP64 energy sums: one block per simulation, fixed order */
-__global__ void batch_energy(const float2* __restrict__ e, const mcxg_simdesc* __restrict__ sims,
-                             double* __restrict__ out) {
-    const mcxg_simdesc& d = sims[blockIdx.x];
+/* per-simulation FP64 energy sums, in an order fixed by the simulation's own
+   threads: row y of the grid is simulation y, its kEnergyParts blocks each sum a
+   stride of them (one block a simulation left 24 of 152 SMs, each with two FP64
+   operations a cycle, to it: 0.54 ms for 2.3 M threads, 0.03 so), then
+   batch_energy_final adds the parts */
+constexpr unsigned int kEnergyParts = 32;
+
+__global__ void __launch_bounds__(256) batch_energy(const float2* __restrict__ e, const mcxg_simdesc* __restrict__ sims,
+                                                    double* __restrict__ part) {
+    const mcxg_simdesc& d = sims[blockIdx.y];
     const unsigned long long base = d.vt_off;
     const unsigned int n = d.kp.nthread;
     double se = 0.0, sl = 0.0;
-    for (unsigned int i = threadIdx.x; i < n; i += blockDim.x) {
+    for (unsigned int i = blockIdx.x * 256u + threadIdx.x; i < n; i += kEnergyParts * 256u) {
         float2 v = e[base + i];
         se += (double)v.x;
         sl += (double)v.y;
@@ -306,7 +358,7 @@ __global__ void batch_energy(const float2* __restrict__ e, const mcxg_simdesc* _
         se += __shfl_down_sync(0xffffffffu, se, o);
         sl += __shfl_down_sync(0xffffffffu, sl, o);
     }
-    __shared__ double wse[32], wsl[32];
+    __shared__ double wse[8], wsl[8];
     if ((threadIdx.x & 31) == 0) {
         wse[threadIdx.x >> 5] = se;
         wsl[threadIdx.x >> 5] = sl;
@@ -314,12 +366,25 @@ __global__ void batch_energy(const float2* __restrict__ e, const mcxg_simdesc* _
     __syncthreads();
     if (threadIdx.x == 0) {
         double a = 0.0, b = 0.0;
-        for (unsigned int w = 0; w < (blockDim.x + 31) / 32; w++) {
+        for (unsigned int w = 0; w < 8; w++) {
             a += wse[w];
             b += wsl[w];
         }
-        out[blockIdx.x * 2] = a;
-        out[blockIdx.x * 2 + 1] = b;
+        double* p = part + 2 * ((size_t)blockIdx.y * kEnergyParts + blockIdx.x);
+        p[0] = a;
+        p[1] = b;
+    }
+}
+
+__global__ void __launch_bounds__(256) batch_energy_final(const double* __restrict__ part, unsigned int nsim,
+                                                          double* __restrict__ out) {
+    for (unsigned int k = blockIdx.x * 256u + threadIdx.x; k < 2u * nsim; k += gridDim.x * 256u) {
+        const double* p = part + 2 * (size_t)(k / 2) * kEnergyParts + (k & 1u);
+        double a = 0.0;
+        for (unsigned int i = 0; i < kEnergyParts; i++) {
+            a += p[2 * i];
+        }
+        out[k] = a;
     }
 }
 
@@ -330,9 +395,7 @@ __global__ void batch_merge(const float* __restrict__ f, unsigned long long tota
     const unsigned long long off = d.field_off;
     const unsigned int n = d.kp.fieldlen;
     const double sc = scales[blockIdx.y];
-    for (unsigned int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        out[off + i] = (float)(cell_value(f, total, (double)d.kp.fxunit, off + i) * sc);
-    }
+    merge_range(f, total, off, n, (double)d.kp.fxunit, [=](size_t) { return sc; }, out);
 }
 
 /* every simulation's compensated field merged in FP64, unscaled */
@@ -836,7 +899,7 @@ int mcxg_destroy(mcxg_session* s) {
                     s->d_detp, s->d_detseed, s->d_words, s->d_events, s->d_red, s->d_out,
                     s->d_rseed, s->d_rweight, s->d_rtof, s->d_rdetid, s->d_scales, s->d_detw,
                     s->d_sims, s->d_simvt, s->d_simctr, s->d_smatrix, s->d_bmedia, s->d_bfield, s->d_benergy, s->d_bsum, s->d_bout,
-                    s->d_adj, s->d_lfib, s->d_jump, s->d_traj, s->d_acc64, s->d_accf, s->d_accs, s->d_adjc,
+                    s->d_adj, s->d_lfib, s->d_lfpow, s->d_jump, s->d_traj, s->d_acc64, s->d_accf, s->d_accs, s->d_adjc,
                     s->d_adjJ, s->d_words32};
     if (s->bgraph_exec) {
         cudaGraphExecDestroy(s->bgraph_exec);
@@ -1046,9 +1109,13 @@ __global__ void __launch_bounds__(128) lfib_words(const uint32_t* __restrict__ s
    map W' = M W (W = o[k-31 .. k-1]; W'[t] = W[t+1] for t < 30, W'[30] =
    W[0] + W[28]), so block j's window is (M^B)^j W0.  lf_powers (one CTA, a
    thread per matrix element, products mod 2^32 in shared memory) makes Q_0 =
-   M^B by square-and-multiply and Q_b = Q_{b-1}^2; lfib_jump_words then
-   applies Q_b to W0 for each set bit b of its block index and expands the
-   block as lfib_words does. */
+   M^B by square-and-multiply and Q_b = Q_{b-1}^2, stored by columns; they
+   depend on B alone and are kept.  A warp of lfib_jump_words takes 32 blocks:
+   lane i holds W[i] and the warp multiplies together, by Q_b for each set bit
+   b >= 5 of its first block's index, then by Q_0 from one block's window to the
+   next; each lane then expands one of the windows as lfib_words does.  (A
+   thread for each block did its 31 x 31 products alone: 151 us for 622,592
+   reference threads' words in blocks of 1,024, 15 us so in blocks of 124.) */
 __device__ __forceinline__ void lf_mul_shared(const uint32_t* X, const uint32_t* Y, uint32_t* Z, int t) {
     uint32_t acc = 0;
     if (t < 31 * 31) {
@@ -1085,7 +1152,7 @@ __global__ void __launch_bounds__(1024) lf_powers(uint32_t blocklen, uint32_t np
     }
     for (uint32_t b = 0; b < npow; b++) {
         if (t < 31 * 31) {
-            pows[31 * 31 * (size_t)b + t] = P[t];
+            pows[31 * 31 * (size_t)b + 31 * (t % 31) + t / 31] = P[t];
         }
         if (b + 1 < npow) {
             lf_mul_shared(P, P, P, t);
@@ -1100,37 +1167,49 @@ __global__ void __launch_bounds__(128) lfib_jump_words(const uint32_t* __restric
        warp then writes lane L's 31 consecutive words with 31 lanes (one
        coalesced run) instead of 32 words 4 x blocklen bytes apart */
     __shared__ uint32_t tile[4][32 * 33];
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    const unsigned int lane = threadIdx.x & 31u;
+    __shared__ uint32_t step[31 * 31];        /* Q_0 */
+    const unsigned int lane = threadIdx.x & 31u, row = lane < 31u ? lane : 30u;
     uint32_t* my = tile[threadIdx.x >> 5];
-    const uint32_t j0 = j - lane;             /* the warp's first block */
+    const uint32_t j0 = (blockIdx.x * blockDim.x + threadIdx.x) - lane;      /* the warp's first block */
+    if (npow) {
+        for (unsigned int t = threadIdx.x; t < 31 * 31; t += blockDim.x) {
+            step[t] = pows[t];
+        }
+    }
+    __syncthreads();
     if (j0 >= nblock) {
         return;                               /* the whole warp is past the last block */
     }
+    uint32_t w = w0[row];
+    for (uint32_t b = 5; b < npow; b++) {
+        if ((j0 >> b) & 1u) {
+            const uint32_t* Q = pows + 31 * 31 * (size_t)b + row;
+            uint32_t acc = 0;
+#pragma unroll
+            for (int m = 0; m < 31; m++) {
+                acc += __ldg(Q + 31 * m) * __shfl_sync(0xFFFFFFFFu, w, m);
+            }
+            w = acc;
+        }
+    }
+    for (unsigned int L = 0; L < 32 && j0 + L < nblock; L++) {
+        if (L) {
+            uint32_t acc = 0;
+#pragma unroll
+            for (int m = 0; m < 31; m++) {
+                acc += step[31 * m + row] * __shfl_sync(0xFFFFFFFFu, w, m);
+            }
+            w = acc;
+        }
+        my[L * 33 + lane] = w;
+    }
+    __syncwarp();
     uint32_t r[31];
 #pragma unroll
     for (int t = 0; t < 31; t++) {
-        r[t] = w0[t];
+        r[t] = my[lane * 33 + t];             /* a lane past the last block expands what it finds, unstored */
     }
-    for (uint32_t b = 0; b < npow; b++) {
-        if (j < nblock && ((j >> b) & 1u)) {
-            const uint32_t* Q = pows + 31 * 31 * (size_t)b;
-            uint32_t w[31];
-#pragma unroll
-            for (int i = 0; i < 31; i++) {
-                uint32_t acc = 0;
-#pragma unroll
-                for (int m = 0; m < 31; m++) {
-                    acc += __ldg(Q + 31 * i + m) * r[m];
-                }
-                w[i] = acc;
-            }
-#pragma unroll
-            for (int i = 0; i < 31; i++) {
-                r[i] = w[i];
-            }
-        }
-    }
+    __syncwarp();
     for (uint32_t off = 0; off < blocklen; off += 31) {
 #pragma unroll
         for (int t = 0; t < 31; t++) {
@@ -1184,9 +1263,9 @@ int mcxg_set_seeds_window(mcxg_session* s, const uint32_t* window, uint32_t nthr
     if (!s || !window || nthread == 0 || nword > 0xFFFFFFFFull) {
         return MCXG_ERR_ARG;
     }
-    /* blocks of at least 1,024 words, at most 65,536 blocks: a 1e8-photon
+    /* blocks of at least 124 words, at most 65,536 blocks: a 1e8-photon
        launch's 80 M words in 65,536 blocks of 1,216 */
-    const uint32_t blocklen = (uint32_t)std::max<uint64_t>(1024, (nword + 65535) / 65536);
+    const uint32_t blocklen = (uint32_t)std::max<uint64_t>(124, (nword + 65535) / 65536);
     const uint32_t nblock = (uint32_t)((nword + blocklen - 1) / blocklen);
     uint32_t npow = 0;
     while (npow < 32 && ((uint64_t)1 << npow) < nblock) {
@@ -1198,19 +1277,28 @@ int mcxg_set_seeds_window(mcxg_session* s, const uint32_t* window, uint32_t nthr
         rc = ensure(&s->d_energy, &s->energy_cap, nthread);
     }
     if (!rc) {
-        rc = ensure(&s->d_lfib, &s->lfib_cap, 31 + 31 * 31 * (size_t)std::max<uint32_t>(npow, 1));
+        rc = ensure(&s->d_lfib, &s->lfib_cap, 31);
+    }
+    const bool kept = s->lfpow_len == blocklen && s->lfpow_n >= npow;
+    if (!rc && !kept) {
+        s->lfpow_len = s->lfpow_n = 0;
+        rc = ensure(&s->d_lfpow, &s->lfpow_cap, 31 * 31 * (size_t)std::max<uint32_t>(npow, 1));
     }
     if (rc) {
         return rc;
     }
     MCXG_TRY(cudaMemcpyAsync(s->d_lfib, window, sizeof(uint32_t) * 31, cudaMemcpyHostToDevice, s->st));
-    if (npow) {
-        lf_powers<<<1, 1024, 0, s->st>>>(blocklen, npow, s->d_lfib + 31);
+    if (npow && !kept) {
+        lf_powers<<<1, 1024, 0, s->st>>>(blocklen, npow, s->d_lfpow);
     }
-    lfib_jump_words<<<(nblock + 127) / 128, 128, 0, s->st>>>(s->d_lfib, s->d_lfib + 31, npow, nblock, blocklen,
+    lfib_jump_words<<<(nblock + 127) / 128, 128, 0, s->st>>>(s->d_lfib, s->d_lfpow, npow, nblock, blocklen,
                                                               (uint32_t)nword, (uint32_t*)s->d_seeds);
     MCXG_TRY(cudaGetLastError());
     MCXG_TRY(cudaStreamSynchronize(s->st));
+    if (!kept) {
+        s->lfpow_len = blocklen;
+        s->lfpow_n = npow;
+    }
     s->has_seeds = true;
     return MCXG_OK;
 }
@@ -1626,7 +1714,7 @@ int mcxg_get_energy(mcxg_session* s, double* escaped, double* launched) {
     }
     MCXG_TRY(cudaSetDevice(s->device));
     energy_partials<<<kRedBlocks, kRedThreads, 0, s->st>>>(s->d_energy, s->kp.nthread, s->d_red);
-    energy_final<<<1, 32, 0, s->st>>>(s->d_red, kRedBlocks);
+    energy_final<<<1, 256, 0, s->st>>>(s->d_red, kRedBlocks);
     double h[2];
     MCXG_TRY(cudaMemcpyAsync(h, s->d_red + 2 * kRedBlocks, sizeof(h), cudaMemcpyDeviceToHost, s->st));
     MCXG_TRY(cudaStreamSynchronize(s->st));
@@ -1659,8 +1747,7 @@ int mcxg_get_field(mcxg_session* s, float* out, double scale) {
     if (rc) {
         return rc;
     }
-    field_merge_f32<<<grid_for(s, total), 256, 0, s->st>>>(s->d_field, n, total, (double)s->kp.fxunit, scale,
-                                                           (float*)s->d_out);
+    field_merge_f32<<<grid_for(s, total), 256, 0, s->st>>>(s->d_field, total, (double)s->kp.fxunit, scale, (float*)s->d_out);
     s->out_valid = true;
     MCXG_TRY(cudaMemcpyAsync(out, s->d_out, sizeof(float) * total, cudaMemcpyDeviceToHost, s->st));
     MCXG_TRY(cudaStreamSynchronize(s->st));
@@ -2062,7 +2149,9 @@ int batch_enqueue(mcxg_session* s, int lflags) {
         a.nsim = n;
         MCXG_TRY(mcxg::batch_launch(a, lflags, s->bt_grid, s->bt_block, s->st));
     }
-    batch_energy<<<s->nsim, 256, 0, s->st>>>(s->d_benergy, s->d_sims, s->d_bsum);
+    double* part = s->d_bsum + 2 * (size_t)s->nsim;
+    batch_energy<<<dim3(kEnergyParts, s->nsim), 256, 0, s->st>>>(s->d_benergy, s->d_sims, part);
+    batch_energy_final<<<(2 * s->nsim + 255) / 256, 256, 0, s->st>>>(part, s->nsim, s->d_bsum);
     return MCXG_OK;
 }
 
@@ -2115,7 +2204,7 @@ int batch_upload(mcxg_session* s, const mcxg_simdesc* sims, uint32_t nsim, const
         rc = ensure(&s->d_benergy, &s->benergy_cap, (size_t)vt);
     }
     if (!rc) {
-        rc = ensure(&s->d_bsum, &s->bsum_cap, 2 * (size_t)nsim);
+        rc = ensure(&s->d_bsum, &s->bsum_cap, 2 * (size_t)nsim * (1 + kEnergyParts));    /* sums, then parts */
     }
     if (rc) {
         return rc;
@@ -2321,7 +2410,7 @@ static int energy_sum_noalloc_on(int device, const float* d_energy, uint32_t nth
     MCXG_TRY(cudaMemsetAsync(scratch, 0, sizeof(double) * (2 * (size_t)nblocks + 2), 0));
     energy_partials<<<nblocks, kRedThreads, 0, 0>>>((const float2*)d_energy, nthread, scratch);
     MCXG_TRY(cudaGetLastError());
-    energy_final<<<1, 32, 0, 0>>>(scratch, (int)nblocks);
+    energy_final<<<1, 256, 0, 0>>>(scratch, (int)nblocks);
     MCXG_TRY(cudaGetLastError());
     MCXG_TRY(cudaMemcpyAsync(d_sums, scratch + 2 * nblocks, 2 * sizeof(double), cudaMemcpyDeviceToDevice, 0));
     MCXG_TRY(cudaStreamSynchronize(0));
