@@ -222,6 +222,8 @@ typedef struct MCXConfig {
     float* exportdebugdata;
     int errorcode;                /* last error in library mode */
     char errormsg[256];
+    int complexpairs;             /* 1: the RF field is exported as {real, imaginary} pairs instead of the reference's
+                                     real plane then imaginary plane */
 } Config;
 
 /* ---- drop-in host interface ------------------------------------------------ */
@@ -505,6 +507,8 @@ int  mcxg_get_thread_energy(mcxg_session* s, float* out);
 /* Field: the compensated accumulator (fixed-point count x unit + remainder) in FP64, times
    scale, rounded to float; fieldlen values. */
 int  mcxg_get_field(mcxg_session* s, float* out, double scale);
+/* A complex (RF) field as fieldlen {real, imaginary} pairs, otherwise as mcxg_get_field. */
+int  mcxg_get_field_pairs(mcxg_session* s, float* out, double scale);
 /* Field split into nblocks equal blocks, block b scaled by scales[b]
    (a replay with one output per detector). */
 int  mcxg_get_field_blocks(mcxg_session* s, float* out, const double* scales, uint32_t nblocks);

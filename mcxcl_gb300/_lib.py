@@ -96,6 +96,7 @@ class Config(ctypes.Structure):
         ("exportdebugdata", ctypes.POINTER(ctypes.c_float)),
         ("errorcode", ctypes.c_int),
         ("errormsg", ctypes.c_char * 256),
+        ("complexpairs", ctypes.c_int),
     ]
 
 
@@ -113,7 +114,7 @@ EXPORTS = [
     "mcx_config_offsetof", "mcx_release_sessions", "mcx_prepare_simulation",
     "mcxg_device_count", "mcxg_device_info", "mcxg_error_string", "mcxg_create", "mcxg_destroy",
     "mcxg_set_problem", "mcxg_set_params", "mcxg_set_seeds", "mcxg_set_seeds_lfib", "mcxg_set_trajectory", "mcxg_get_trajectory", "mcxg_set_launch", "mcxg_simulate",
-    "mcxg_get_energy", "mcxg_get_thread_energy", "mcxg_get_field", "mcxg_get_field_f64", "mcxg_get_detected",
+    "mcxg_get_energy", "mcxg_get_thread_energy", "mcxg_get_field", "mcxg_get_field_pairs", "mcxg_get_field_f64", "mcxg_get_detected",
     "mcxg_get_counters", "mcxg_get_launch", "mcxg_fp32_peak", "mcxg_energy_sum_noalloc", "mcxg_autotune",
     "mcxg_set_replay", "mcxg_get_field_blocks", "mcxg_get_field_interleaved", "mcxg_set_polarization", "mcx_mie", "mcxg_get_detweight", "mcx_run_batch", "mcxg_batch_set",
     "mcxg_batch_simulate", "mcxg_batch_get_energy", "mcxg_batch_get_field", "mcx_savedetphoton",
@@ -183,6 +184,7 @@ def load():
     L.mcxg_get_energy.argtypes = [vp, P(ctypes.c_double), P(ctypes.c_double)]
     L.mcxg_get_thread_energy.argtypes = [vp, vp]
     L.mcxg_get_field.argtypes = [vp, vp, ctypes.c_double]
+    L.mcxg_get_field_pairs.argtypes = [vp, vp, ctypes.c_double]
     L.mcxg_get_field_f64.argtypes = [vp, vp]
     L.mcxg_get_verify.argtypes = [vp, vp, vp, vp]
     L.mcxg_get_field_planes.argtypes = [vp, vp, vp]

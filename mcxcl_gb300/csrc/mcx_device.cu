@@ -305,6 +305,30 @@ __global__ void field_merge_f32(const float* __restrict__ f, size_t total, doubl
     merge_range(f, total, 0, total, unit, [=](size_t) { return scale; }, out);
 }
 
+/* a complex field's two components as pairs */
+__global__ void field_merge_pairs(const float* __restrict__ f, size_t n, double unit, double scale, float2* __restrict__ out) {
+    const long long* hi = reinterpret_cast<const long long*>(f);
+    const float* lo = f + 4 * n;
+    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += 2 * stride) {
+        long long k[4];
+        float r[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const size_t j = i + (u >> 1) * stride;
+            k[u] = j < n ? __ldcs(hi + (u & 1) * n + j) : 0ll;
+            r[u] = j < n ? __ldcs(lo + (u & 1) * n + j) : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u += 2) {
+            const size_t j = i + (u >> 1) * stride;
+            if (j < n) {
+                out[j] = make_float2(merged_f32(k[u], r[u], unit, scale), merged_f32(k[u + 1], r[u + 1], unit, scale));
+            }
+        }
+    }
+}
+
 /* element j belongs to source j % nsrc (photon sharing interleaves the
    patterns innermost) */
 __global__ void field_merge_interleaved(const float* __restrict__ f, size_t n, size_t total, double unit,
@@ -1750,6 +1774,24 @@ int mcxg_get_field(mcxg_session* s, float* out, double scale) {
     field_merge_f32<<<grid_for(s, total), 256, 0, s->st>>>(s->d_field, total, (double)s->kp.fxunit, scale, (float*)s->d_out);
     s->out_valid = true;
     MCXG_TRY(cudaMemcpyAsync(out, s->d_out, sizeof(float) * total, cudaMemcpyDeviceToHost, s->st));
+    MCXG_TRY(cudaStreamSynchronize(s->st));
+    return MCXG_OK;
+}
+
+int mcxg_get_field_pairs(mcxg_session* s, float* out, double scale) {
+    if (!s || !out || !s->has_problem || field_comps(s->kp) != 2) {
+        return MCXG_ERR_ARG;
+    }
+    MCXG_TRY(cudaSetDevice(s->device));
+    const size_t n = s->kp.fieldlen;
+    int rc = ensure((double**)&s->d_out, &s->out_cap, 2 * n);
+    if (rc) {
+        return rc;
+    }
+    field_merge_pairs<<<grid_for(s, n), 256, 0, s->st>>>(s->d_field, n, (double)s->kp.fxunit, scale, (float2*)s->d_out);
+    s->out_valid = false;
+    MCXG_TRY(cudaGetLastError());
+    MCXG_TRY(cudaMemcpyAsync(out, s->d_out, sizeof(float) * 2 * n, cudaMemcpyDeviceToHost, s->st));
     MCXG_TRY(cudaStreamSynchronize(s->st));
     return MCXG_OK;
 }

@@ -1865,6 +1865,8 @@ static void run_simulation(Config* cfg) {
             device_check(mcxg_get_field_interleaved(s, dst, blockscale, nblocks), "reading the field");
         } else if (blockscale) {
             device_check(mcxg_get_field_blocks(s, dst, blockscale, nblocks), "reading the field");
+        } else if (cfg->complexpairs && cfg->omega > 0.f && !replay) {     /* never with shared photons */
+            device_check(mcxg_get_field_pairs(s, dst, scale), "reading the field");
         } else {
             device_check(mcxg_get_field(s, dst, scale), "reading the field");
         }
@@ -2224,7 +2226,7 @@ static const struct {
     MCX_FIELD(failedlaunch), MCX_FIELD(threadused), MCX_FIELD(exportenergy), MCX_FIELD(savethreadenergy),
     MCX_FIELD(autotune), MCX_FIELD(savedetweight), MCX_FIELD(exportdetweight), MCX_FIELD(replaysiteown), MCX_FIELD(omega),
     MCX_FIELD(polprop), MCX_FIELD(polmedianum), {"lambda_", offsetof(Config, lambda)}, MCX_FIELD(srciquv),
-    MCX_FIELD(smatrix), MCX_FIELD(maxjumpdebug), MCX_FIELD(debugdatalen), MCX_FIELD(exportdebugdata), MCX_FIELD(errorcode), MCX_FIELD(errormsg),
+    MCX_FIELD(smatrix), MCX_FIELD(maxjumpdebug), MCX_FIELD(debugdatalen), MCX_FIELD(exportdebugdata), MCX_FIELD(errorcode), MCX_FIELD(errormsg), MCX_FIELD(complexpairs),
 };
 
 size_t mcx_config_sizeof(void) {

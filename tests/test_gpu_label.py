@@ -146,3 +146,27 @@ def test_batch_as_the_general_kernel(per_thread):
         assert x["stat"]["energytot"] == y["stat"]["energytot"] and x["stat"]["energyabs"] == y["stat"]["energyabs"]
         f, g = np.asarray(x["flux"], np.float64), np.asarray(y["flux"], np.float64)
         assert np.linalg.norm(g) > 0 and np.linalg.norm(f - g) <= 1e-6 * np.linalg.norm(g)
+
+
+@pytest.mark.parametrize("extra", [{}, cases.VARIANTS["multisrc_id"], _ODD])
+def test_complex_pairs_hold_the_planes(extra):
+    """run()'s complex field, exported as pairs, against the two planes the C interface exports by default."""
+    import ctypes
+
+    import mcxcl_gb300
+    from mcxcl_gb300 import _lib, pmcxcl
+    cfg = cases.small_two_media(**dict(dict(nphoton=20000, omega=2 * np.pi * 1e8), **extra))
+    flux = mcxcl_gb300.run(cfg)["flux"]
+    L, C = _lib.load(), _lib.Config()
+    try:
+        pmcxcl.parse_config(cfg, C)
+        L.mcx_validatecfg(ctypes.byref(C), None, None, 0)
+        L.mcx_run_simulation(ctypes.byref(C), None, None)
+        pmcxcl._check(C)
+        planes = np.ctypeslib.as_array(C.exportfield, shape=(2 * flux.size,)).copy()
+    finally:
+        L.mcx_clearcfg(ctypes.byref(C))
+    assert flux.dtype == np.complex64 and flux.flags["F_CONTIGUOUS"] and np.abs(planes[flux.size:]).max() > 0
+    want = (planes[:flux.size] + 1j * planes[flux.size:]).reshape(flux.shape, order="F")
+    # two runs of the same photons: the order of the remainders' float sums
+    assert np.abs(flux - want).max() <= 1e-6 * np.abs(want).max()
