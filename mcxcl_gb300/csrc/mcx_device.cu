@@ -1683,12 +1683,23 @@ int mcxg_autotune(mcxg_session* s, uint32_t sample_photons, int* block, int* blo
         int block, bpsm, noagg;
     } cands[] = {{256, 4, 1}, {128, 8, 1}, {64, 16, 1}, {256, 2, 1}, {128, 4, 1}, {0, 0, 0}};
     const int ncand = (int)(sizeof(cands) / sizeof(cands[0]));
+    /* the usual configurations' kernel runs blocks of 256 in one register
+       budget; how many a SM follows from the whole run's photons (shape_for), as
+       a sample, mostly tail, always favours few */
+    const bool label = label_run(full, 0u) >= 0 && !s->npol && !s->maxjump;
+    if (label) {
+        unsigned int lanes = 32;
+        shape_for(total, s->info.sm, true, &cands[0].bpsm, &lanes);
+    }
     float best = 1e30f;
     Cand pick = cands[0];
     int keep_block = s->block_req, keep_bpsm = s->bpsm_req;
     int rc = MCXG_OK;
     for (int ci = 0; ci < ncand && !rc; ci++) {
         Cand c = cands[ci];
+        if (label && ci && c.block == 256) {
+            continue;
+        }
         if (!c.block) {
             c = pick;            /* the last candidate: the best shape, aggregated */
             c.noagg = 0;
