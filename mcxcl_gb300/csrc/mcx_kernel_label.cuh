@@ -10,19 +10,19 @@
  *
  * The kernel is bound by issue: a warp runs the scattering and the
  * voxel-crossing block in nearly every iteration, each with about half its
- * lanes, so the instructions of an iteration are what counts.  One of the
- * cube + sphere workload's took 550 (counted by ncu) and takes 300: no tests of what is
- * fixed; nothing but deposits, label and voxel index for the lanes that
- * cross a face, and what is rare (faces of the domain, label changes,
- * time-outs, roulette) behind one test; conditions combined without
- * branches; voxel coordinates as floats; the parameters of a step in four
- * vector loads; a deposit scale per label instead of a choice of output;
- * what a replayed photon deposits looked up once, at its launch.
- * Kernel times before and after at the same launch shape (one GB300): cube,
- * 1e6 photons 8.95 -> 6.0 ms; cube + sphere with detectors, 1e6 14.1 -> 8.9 ms, 2e7
- * 113 -> 79 ms; head, 1e7 42.9 -> 32 ms.  Calls: modulated sphere 1e6 18.0 -> 10.2 ms,
- * replay of 9,000 photons 4.9 -> 3.1 ms, readings and their gradient on a
- * 100^3 absorption map 23.5 -> 14.6 ms, fluence gradient 47 -> 39 ms.
+ * lanes, so the instructions of an iteration are what counts.  The cube +
+ * sphere workload took 5,825 warp instructions a photon (counted by ncu) and
+ * takes 3,780: no tests of what is fixed; nothing but deposits, label and
+ * voxel index for the lanes that cross a face, and what is rare (faces of the
+ * domain, label changes, time-outs, roulette) behind one test; conditions
+ * combined without branches; voxel coordinates as floats; the parameters of a
+ * step in four vector loads; a deposit scale per label instead of a choice of
+ * output; what a replayed photon deposits looked up once, at its launch.
+ * Kernel times before and after (one GB300; the small runs also by their
+ * launch shape): cube, 1e4 photons 2.66 -> 1.23 ms, 1e6 8.95 -> 4.4 ms; cube +
+ * sphere with detectors, 1e6 14.1 -> 7.1 ms, 2e7 113 -> 75 ms; head, 1e7 42.9 ->
+ * 29 ms; modulated sphere, 1e6 17.2 -> 8.6 ms; replay of 9,000 photons 4.7 -> 1.75
+ * ms; 1e6 photons on a 100^3 absorption map 13.3 -> 6.9 ms.
  */
 #ifndef MCX_KERNEL_LABEL_CUH
 #define MCX_KERNEL_LABEL_CUH
