@@ -1588,8 +1588,11 @@ int mcxg_simulate(mcxg_session* s, unsigned int flags, float* kernel_ms) {
         }
     }
     /* the usual configurations have a kernel of their own */
-    const int lrun = (exact || pol || svmc || xmedia || s->maxjump || (flags & MCXG_GENERAL) || block != mcxg::kLabelBlock ||
+    int lrun = (exact || pol || svmc || xmedia || s->maxjump || (flags & MCXG_GENERAL) || block != mcxg::kLabelBlock ||
                       (lflags & (mcxg::LF_WAGG | mcxg::LF_TILE | mcxg::LF_ACC64))) ? -1 : label_run(kp, adjmode);
+    if (lrun >= 0 && label_shared_bytes(kp) > s->info.sharedmem_per_block) {
+        lrun = -1;         /* a slot more for each kind of record: the last media that fit the other kernel's layout */
+    }
     const bool label = lrun >= 0;
     if (label) {
         lflags |= (kp.mediaformat == 101 ? mcxg::LF_MUA : 0) | lrun << mcxg::LF_RUN |

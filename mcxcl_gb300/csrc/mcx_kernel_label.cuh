@@ -387,7 +387,7 @@ __device__ __forceinline__ Replayed replayed(const KArgs& a, const PS& ps, unsig
    ms with the lane's index held in a register, head 1e7 31.2 -> 29.8; other
    sources' runs 2 % slower for the code between). */
 __device__ __forceinline__ bool plainbeam(const mcxg_kparams& c_p) {
-    return c_p.srctype == S_PENCIL && !c_p.nangle && c_p.srcdir.w == 0.f && !c_p.replay && c_p.maxvoidstep >= 1u &&
+    return c_p.srctype == S_PENCIL && !c_p.nangle && c_p.srcdir.w == 0.f && !c_p.replay && c_p.maxvoidstep >= 2u &&
            (__float_as_uint(c_p.srcparam2.w) & K_MED_MASK) && fabsf(c_p.srcpos.w) > c_p.minenergy;
 }
 

@@ -42,7 +42,12 @@ CASES = {
     "one voxel": cases.VARIANTS["onevoxel"], "few photons": dict(nphoton=100), "specular": cases.VARIANTS["outside_src_specular"],
     "wide label": dict(vol=np.full((40, 40, 40), 127, np.uint8), prop=[[0, 0, 1, 1]] + [[0.01, 1, 0.5, 1.37]] * 127, savedetflag="d"),
     "angles": cases.VARIANTS["angleinvcdf"], "pattern": cases.VARIANTS["pattern"], "isotropic": cases.VARIANTS["isotropic"],
-    "many gates": dict(tstep=2e-11), "backward": dict(prop=[[0, 0, 1, 1], [0.01, 2, -0.4, 1.37], [0.02, 5, 0.87, 1.45]]),
+    "many gates": dict(tstep=2e-11), "one void step": dict(maxvoidstep=1), "two void steps": dict(maxvoidstep=2),
+    # the most media whose records fit the general kernel's shared memory, and some fewer
+    "72 media": dict(vol=np.arange(1, 41, dtype=np.uint8)[:, None, None] + np.zeros((1, 40, 40), np.uint8), savedetflag="dspm",
+                     prop=[[0, 0, 1, 1]] + [[0.01, 1, 0.5, 1.37]] * 71),
+    "60 media": dict(vol=np.arange(1, 41, dtype=np.uint8)[:, None, None] + np.zeros((1, 40, 40), np.uint8), savedetflag="dspm",
+                     prop=[[0, 0, 1, 1]] + [[0.01, 1, 0.5, 1.37]] * 59), "backward": dict(prop=[[0, 0, 1, 1], [0.01, 2, -0.4, 1.37], [0.02, 5, 0.87, 1.45]]),
     # float absorption: voxels without any, and every record kind
     "mua": dict(_MUA, savedetflag="dxv"), "mua energy": dict(_MUA, outputtype="energy"), "mua plain": dict(_MUA, issavedet=0, issaveseed=0),
     "mua matched": dict(_MUA, isreflect=0, savedetflag="dspm", minenergy=0.01), "mua gates": dict(_MUA, tstart=1e-10, tend=1.7e-9, tstep=1e-10),
