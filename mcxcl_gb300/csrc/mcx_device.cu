@@ -951,11 +951,24 @@ int mcxg_destroy(mcxg_session* s) {
 
 namespace {
 /* 32-bit label words (label | detector bit 31) to the kernel's bytes (label |
-   detector bit 7, the bits of keep), labels below 128 */
-__global__ void pack_labels(const uint32_t* __restrict__ words, size_t n, uint32_t keep, uint8_t* __restrict__ bytes) {
+   detector bit 7, the bits of keep), labels below 128; bounded by the last
+   medium, which the transport kernel's tables and record slots rely on (the
+   host driver has refused larger ones before) */
+__global__ void pack_labels(const uint32_t* __restrict__ words, size_t n, uint32_t keep, uint32_t last,
+                            uint8_t* __restrict__ bytes) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const uint32_t w = words[i];
-        bytes[i] = (uint8_t)(((w & 0x7Fu) | ((w >> 24) & 0x80u)) & keep);
+        bytes[i] = (uint8_t)((min(w & 0x7Fu, last) | ((w >> 24) & 0x80u)) & keep);
+    }
+}
+
+/* the same bound on labels uploaded as bytes */
+__global__ void bound_labels(uint8_t* __restrict__ bytes, size_t n, uint32_t last) {
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        const uint32_t b = bytes[i];
+        if ((b & 0x7Fu) > last) {
+            bytes[i] = (uint8_t)(last | (b & 0x80u));
+        }
     }
 }
 }  // namespace
@@ -1028,10 +1041,15 @@ int mcxg_set_problem(mcxg_session* s, const void* kparams, size_t kparams_size, 
     }
     if (pack) {
         MCXG_TRY(cudaMemcpyAsync(s->d_words32, media, sizeof(uint32_t) * (size_t)kp.nvox, cudaMemcpyHostToDevice, s->st));
-        pack_labels<<<grid_for(s, kp.nvox), 256, 0, s->st>>>(s->d_words32, kp.nvox, 0xFFu, (uint8_t*)s->d_media);
+        pack_labels<<<grid_for(s, kp.nvox), 256, 0, s->st>>>(s->d_words32, kp.nvox, 0xFFu, kp.medianum - 1u,
+                                                             (uint8_t*)s->d_media);
         MCXG_TRY(cudaGetLastError());
     } else {
         MCXG_TRY(cudaMemcpyAsync(s->d_media, media, mbytes, cudaMemcpyHostToDevice, s->st));
+        if (mediaword == 1 && kp.medianum) {
+            bound_labels<<<grid_for(s, kp.nvox), 256, 0, s->st>>>((uint8_t*)s->d_media, kp.nvox, kp.medianum - 1u);
+            MCXG_TRY(cudaGetLastError());
+        }
     }
     MCXG_TRY(cudaMemcpyAsync(s->d_prop, prop, sizeof(float) * 4 * kp.medianum, cudaMemcpyHostToDevice, s->st));
     if (kp.nphase) {
@@ -2275,10 +2293,13 @@ int batch_upload(mcxg_session* s, const mcxg_simdesc* sims, uint32_t nsim, const
         }
         /* a batch saves no detected photons: the label alone, as the byte upload takes it */
         pack_labels<<<grid_for(s, (size_t)nmedia), 256, 0, s->st>>>(s->d_words32, (size_t)nmedia, 0x7Fu,
-                                                                     (uint8_t*)s->d_bmedia);
+                                                                     MCXG_BATCH_MAXMEDIA - 1u, (uint8_t*)s->d_bmedia);
         MCXG_TRY(cudaGetLastError());
     } else {
         MCXG_TRY(cudaMemcpyAsync(s->d_bmedia, media, (size_t)nmedia, cudaMemcpyHostToDevice, s->st));
+        bound_labels<<<grid_for(s, (size_t)nmedia), 256, 0, s->st>>>((uint8_t*)s->d_bmedia, (size_t)nmedia,
+                                                                      MCXG_BATCH_MAXMEDIA - 1u);
+        MCXG_TRY(cudaGetLastError());
     }
     batch_recip<<<grid_for(s, (size_t)nsim * MCXG_BATCH_MAXMEDIA), 256, 0, s->st>>>(s->d_sims, nsim);
     MCXG_TRY(cudaStreamSynchronize(s->st));

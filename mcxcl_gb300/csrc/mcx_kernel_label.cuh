@@ -483,7 +483,9 @@ __global__ void __launch_bounds__(LB_BLOCK, KIND == RUN_RF ? 3 : 4) mcx_transpor
                     st = RUNNING;
                     nsteps = 0;
                     offgrid = true;
-                    m = VOL == VOL_MUA ? s.mediaid : (s.mediaid & V::kMedium) | ((s.mediaid & K_DET_MASK) >> 24);
+                    /* a point source's voxel value comes from the host: bounded as the volume's are */
+                    m = VOL == VOL_MUA ? s.mediaid : min(s.mediaid & V::kMedium, PS::kBatch ? MCXG_BATCH_MAXMEDIA - 1u : c_p.maxmedia) |
+                        ((s.mediaid & K_DET_MASK) >> 24);
                     if (JAC || SITE) {
                         rp = replayed<KIND>(a, ps, vt, s.f.w);
                     }
