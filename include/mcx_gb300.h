@@ -588,6 +588,9 @@ int  mcxg_fp32_peak(mcxg_session* s, double* gops);
 int  mcxg_energy_sum_noalloc(int device, const float* d_energy, uint32_t nthread, double* d_sums);
 /* The persistent grid actually used by the last launch. */
 int  mcxg_get_launch(mcxg_session* s, int* grid, int* block, int* regs);
+/* Which transport kernel the last mcxg_simulate or mcxg_batch_simulate ran: 1
+   the usual configurations' (mcx_kernel_label.cuh), 0 the general one. */
+int  mcxg_get_kernel(mcxg_session* s, int* usual);
 
 #ifdef __cplusplus
 }

@@ -115,7 +115,7 @@ EXPORTS = [
     "mcxg_device_count", "mcxg_device_info", "mcxg_error_string", "mcxg_create", "mcxg_destroy",
     "mcxg_set_problem", "mcxg_set_params", "mcxg_set_seeds", "mcxg_set_seeds_lfib", "mcxg_set_trajectory", "mcxg_get_trajectory", "mcxg_set_launch", "mcxg_simulate",
     "mcxg_get_energy", "mcxg_get_thread_energy", "mcxg_get_field", "mcxg_get_field_pairs", "mcxg_get_field_f64", "mcxg_get_detected",
-    "mcxg_get_counters", "mcxg_get_launch", "mcxg_fp32_peak", "mcxg_energy_sum_noalloc", "mcxg_autotune",
+    "mcxg_get_counters", "mcxg_get_launch", "mcxg_get_kernel", "mcxg_fp32_peak", "mcxg_energy_sum_noalloc", "mcxg_autotune",
     "mcxg_set_replay", "mcxg_get_field_blocks", "mcxg_get_field_interleaved", "mcxg_set_polarization", "mcx_mie", "mcxg_get_detweight", "mcx_run_batch", "mcxg_batch_set",
     "mcxg_batch_simulate", "mcxg_batch_get_energy", "mcxg_batch_get_field", "mcx_savedetphoton",
     "mcxg_adjoint", "mcxg_get_verify", "mcx_readconfig", "mcx_parsejson", "mcxg_adjoint_field",
@@ -195,6 +195,7 @@ def load():
     L.mcxg_get_detected.argtypes = [vp, vp, vp, P(ctypes.c_uint32)]
     L.mcxg_get_counters.argtypes = [vp, vp, vp]
     L.mcxg_get_launch.argtypes = [vp, P(ctypes.c_int), P(ctypes.c_int), P(ctypes.c_int)]
+    L.mcxg_get_kernel.argtypes = [vp, P(ctypes.c_int)]
     L.mcxg_fp32_peak.argtypes = [vp, P(ctypes.c_double)]
     L.mcxg_energy_sum_noalloc.argtypes = [ctypes.c_int, vp, ctypes.c_uint32, vp]
     L.mcxg_autotune.argtypes = [vp, ctypes.c_uint32, P(ctypes.c_int), P(ctypes.c_int), P(ctypes.c_int)]

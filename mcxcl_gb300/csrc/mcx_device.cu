@@ -144,7 +144,7 @@ struct mcxg_session {
     mcxg::KArgs::Tile tile_used{};   /* the last launch's tile (nx = 0: none) */
     int tuned = 0;                   /* 1 once mcxg_autotune picked a shape for this problem */
     int tuned_noagg = 0;
-    int grid = 0, block = 0, regs = 0;
+    int grid = 0, block = 0, regs = 0, usual = 0;
 };
 
 namespace {
@@ -597,19 +597,14 @@ void shape_for(unsigned long long photons, int sms, bool label, int* blocks, uns
    volumes of byte labels or float absorption with one Henyey-Greenstein source
    and no scattering count at which g drops to 0 (a float count of scatterings
    stops below 2^24 + 1), voxel indices of 15 bits; deposits of flux, fluence
-   or energy, the replays that deposit path or scatterings, modulated sources
-   in label volumes, and the first pass of the fluence gradient */
-int label_run(const mcxg_kparams& kp, unsigned int adjmode) {
+   or energy, the replays that deposit path or scatterings, and modulated
+   sources in label volumes */
+int label_run(const mcxg_kparams& kp) {
     const bool labels = kp.mediaword == 1 && kp.mediaformat <= 4;
     const bool mua = kp.mediaformat == 101 && kp.mediaword == 4 && kp.medianum >= 2;
     if (!(labels || mua) || kp.is2d || kp.nphase > 2 || kp.srcnum > 1 || !kp.save2pt || kp.extrasrclen ||
             kp.gscatter <= (1u << 24) || kp.dimx > 32767u || kp.dimy > 32767u || kp.dimz > 32767u) {
         return -1;
-    }
-    if (adjmode) {
-        /* the second pass stays where it was: its float sums drop up to 1e-4 of the
-           hottest voxels' gradients, how much depends on the order of the additions */
-        return adjmode == 1u ? mcxg::RUN_ADJ1 : -1;
     }
     if (kp.omega > 0.f && !kp.replay) {
         return labels ? mcxg::RUN_RF : -1;
@@ -1606,12 +1601,19 @@ int mcxg_simulate(mcxg_session* s, unsigned int flags, float* kernel_ms) {
         }
     }
     /* the usual configurations have a kernel of their own */
-    int lrun = (exact || pol || svmc || xmedia || s->maxjump || (flags & MCXG_GENERAL) || block != mcxg::kLabelBlock ||
-                      (lflags & (mcxg::LF_WAGG | mcxg::LF_TILE | mcxg::LF_ACC64))) ? -1 : label_run(kp, adjmode);
+    /* The gradient's passes stay on the general kernel.  The second one's float
+       sums drop up to 1e-4 of the hottest voxels' gradients, how much depends on
+       the order of the additions; the first one's totals are the same to the bit on
+       either kernel, but with another kernel before it the second pass starts out
+       of step and its order varies more (two calls' dL/dmus 5.7e-6 apart on
+       average, 3.7 to 4.1e-6 with its own kernel before it; 1e6 photons, 60^3) */
+    int lrun = (exact || pol || svmc || xmedia || s->maxjump || adjmode || (flags & MCXG_GENERAL) || block != mcxg::kLabelBlock ||
+                      (lflags & (mcxg::LF_WAGG | mcxg::LF_TILE | mcxg::LF_ACC64))) ? -1 : label_run(kp);
     if (lrun >= 0 && label_shared_bytes(kp) > s->info.sharedmem_per_block) {
         lrun = -1;         /* a slot more for each kind of record: the last media that fit the other kernel's layout */
     }
     const bool label = lrun >= 0;
+    s->usual = label;
     if (label) {
         lflags |= (kp.mediaformat == 101 ? mcxg::LF_MUA : 0) | lrun << mcxg::LF_RUN |
                   (int)(kp.savedetflag & 0xEu) << mcxg::LF_KINDS;
@@ -1707,7 +1709,7 @@ int mcxg_autotune(mcxg_session* s, uint32_t sample_photons, int* block, int* blo
     /* the usual configurations' kernel runs blocks of 256 in one register
        budget; how many a SM follows from the whole run's photons (shape_for), as
        a sample, mostly tail, always favours few */
-    const bool label = label_run(full, 0u) >= 0 && !s->npol && !s->maxjump;
+    const bool label = label_run(full) >= 0 && !s->npol && !s->maxjump;
     if (label) {
         unsigned int lanes = 32;
         shape_for(total, s->info.sm, true, &cands[0].bpsm, &lanes);
@@ -2342,7 +2344,7 @@ int mcxg_batch_simulate(mcxg_session* s, unsigned int flags, float* kernel_ms) {
     for (const mcxg_simdesc& d : s->h_sims) {
         refl = refl || d.kp.dorefl_compiled;
         common = common && !d.kp.is2d && d.kp.mediaformat <= 4 && d.kp.nphase <= 2;
-        label = label && label_run(d.kp, 0u) == mcxg::RUN_FWD;
+        label = label && label_run(d.kp) == mcxg::RUN_FWD;
     }
     const bool verify = (flags & MCXG_VERIFY) != 0;
     if (verify) {
@@ -2373,6 +2375,7 @@ int mcxg_batch_simulate(mcxg_session* s, unsigned int flags, float* kernel_ms) {
     if (label && !agg && !verify && !(flags & MCXG_GENERAL) && block == mcxg::kLabelBlock) {
         lflags |= mcxg::LF_LABEL;
     }
+    s->usual = (lflags & mcxg::LF_LABEL) != 0;
     int occ = 0;
     MCXG_TRY(mcxg::batch_occupancy(lflags, block, std::min<uint32_t>(s->nsim, mcxg::kBatchWave), &occ));
     int bpsm = std::max(1, std::min(bpsm_req, occ > 0 ? occ : bpsm_req));
@@ -2524,6 +2527,14 @@ int mcxg_get_launch(mcxg_session* s, int* grid, int* block, int* regs) {
     if (regs) {
         *regs = s->regs;
     }
+    return MCXG_OK;
+}
+
+int mcxg_get_kernel(mcxg_session* s, int* usual) {
+    if (!s || !usual) {
+        return MCXG_ERR_ARG;
+    }
+    *usual = s->usual;
     return MCXG_OK;
 }
 

@@ -44,8 +44,6 @@ static void* kvol(int flags) {
         return kany<RUN_JAC, VOL>(flags);
     case RUN_SITE:
         return kany<RUN_SITE, VOL>(flags);
-    case RUN_ADJ1:
-        return krefl<RUN_ADJ1, VOL, DET_NONE>(flags);
     }
     if (!(flags & LF_DET)) {
         return krefl<RUN_FWD, VOL, DET_NONE>(flags);

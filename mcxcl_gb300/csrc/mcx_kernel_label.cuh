@@ -2,9 +2,8 @@
  * mcx_kernel_label.cuh -- the transport kernel of the usual configurations.
  *
  * Byte labels or float absorption, three dimensions, Henyey-Greenstein, one
- * source; deposits of flux, fluence or energy, replays, modulated sources
- * and the first pass of the fluence gradient -- each with all of that fixed at
- * compile time.  The photons, their random numbers and every
+ * source; deposits of flux, fluence or energy, replays and modulated sources
+ * -- each with all of that fixed at compile time.  The photons, their random numbers and every
  * rounding are those of mcx_transport (mcx_kernel.cuh), whose device
  * functions it shares; what differs is what a step costs.
  *
@@ -294,8 +293,8 @@ __device__ __forceinline__ float sign1(float x) {
    compiler contracts them in mcx_transport, where a run of these
    configurations went before and some still go (other launch shapes,
    aggregated deposits): the photons stay the same to the bit.  GEN: as in the
-   general instantiations, which float absorption, modulated sources and the
-   fluence gradient took, rather than the common ones.  There the square of g
+   general instantiations, which float absorption and modulated sources took,
+   rather than the common ones.  There the square of g
    and of the quotient are rounded by themselves, and the rotation's y starts
    from the other product. */
 template <bool GEN>
@@ -422,8 +421,8 @@ template <int KIND, int VOL, int DET, bool REFL>
 __global__ void __launch_bounds__(LB_BLOCK, KIND == RUN_RF ? 3 : 4) mcx_transport_label(const KArgs a) {
     typedef Mth<false> M;
     typedef Voxel<VOL> V;
-    constexpr bool GEN = VOL == VOL_MUA || KIND == RUN_RF || KIND == RUN_ADJ1;
-    constexpr bool JAC = KIND == RUN_JAC, SITE = KIND == RUN_SITE, RF = KIND == RUN_RF, ADJ = KIND == RUN_ADJ1;
+    constexpr bool GEN = VOL == VOL_MUA || KIND == RUN_RF;
+    constexpr bool JAC = KIND == RUN_JAC, SITE = KIND == RUN_SITE, RF = KIND == RUN_RF;
     typedef LabelPS<VOL, DET> PS;
     PS ps;
     Shared S;
@@ -443,16 +442,12 @@ __global__ void __launch_bounds__(LB_BLOCK, KIND == RUN_RF ? 3 : 4) mcx_transpor
     bool offgrid = false;
     s.f.x = 1.f;
     Replayed rp = {0.f, 1.f, 0u};
-    float adjJ = 0.f;                      /* fluence gradient: the photon's loss total */
     int st = (threadIdx.x & 31u) < a.lanes ? ps.claim(a, vt) : DONE;
 
     while (__any_sync(0xFFFFFFFFu, st != DONE)) {
         if (st == ENDED || st == FRESH) {
             const mcxg_kparams& c_p = ps.p();
             bool go = true;
-            if (ADJ && st == ENDED) {
-                a.adjJ[adj_slot(c_p, vt, s.f.w)] = adjJ;
-            }
             if (st == ENDED && closephoton<DET != DET_NONE, false, false>(a, ps, S, s, endflag, vt)) {
                 a.energy[ps.vt_off() + vt] = make_float2(ps.cold()->esc, ps.cold()->launched);
                 st = ps.claim(a, vt);
@@ -489,7 +484,6 @@ __global__ void __launch_bounds__(LB_BLOCK, KIND == RUN_RF ? 3 : 4) mcx_transpor
                     if (JAC || SITE) {
                         rp = replayed<KIND>(a, ps, vt, s.f.w);
                     }
-                    adjJ = 0.f;
                     cx = (float)s.fx + 0.5f;
                     cy = (float)s.fy + 0.5f;
                     cz = (float)s.fz + 0.5f;
@@ -638,14 +632,7 @@ __global__ void __launch_bounds__(LB_BLOCK, KIND == RUN_RF ? 3 : 4) mcx_transpor
                         const float4 C = ps.row(label, 2);
                         weight = C.z > 0.f ? __fmul_rn(s.w0, s.pathlen) : __fmul_rn(__fsub_rn(s.w0, s.p.w), C.y);
                     }
-                    if (ADJ) {
-                        if (left) {
-                            const bool dep = inwin & (fabsf(weight) > 0.f);
-                            /* the visit that just ended, in voxel idxold */
-                            const float c = dep ? __ldg(a.adjc + key) : 0.f;
-                            adjJ = __fadd_rn(adjJ, __fmul_rn(c, weight));
-                        }
-                    } else if (left & (s.f.y >= h1.z) & (s.f.y < h1.x) & (fabsf(weight) > 0.f)) {
+                    if (left & (s.f.y >= h1.z) & (s.f.y < h1.x) & (fabsf(weight) > 0.f)) {
                         /* field_split and field_commit: the rounded product is a float
                            integer, the remainder one exact fma */
                         const float kf = rintf(__fmul_rn(weight, h2.x));
