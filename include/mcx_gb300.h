@@ -222,8 +222,6 @@ typedef struct MCXConfig {
     float* exportdebugdata;
     int errorcode;                /* last error in library mode */
     char errormsg[256];
-    int complexpairs;             /* 1: the RF field is exported as {real, imaginary} pairs instead of the reference's
-                                     real plane then imaginary plane */
 } Config;
 
 /* ---- drop-in host interface ------------------------------------------------ */
@@ -267,6 +265,10 @@ void mcx_cleargpuinfo(GPUInfo** info);
    The calling thread's current CUDA device is the same on return as before
    (the run itself uses the device cfg selects). */
 void mcx_run_simulation(Config* cfg, float* fluence, float* totalenergy);
+/* The same, except that a modulated source's field (omega > 0, no replay) is
+   exported as {real, imaginary} pairs instead of the reference's real plane
+   then imaginary plane. */
+void mcx_run_simulation_pairs(Config* cfg);
 /* Frees one output buffer that a caller took over from cfg (exportfield,
    exportdetected, seeddata, ...: set the Config's pointer to NULL first so
    mcx_clearcfg leaves it alone).  While sessions are kept (mcx_keep_sessions,

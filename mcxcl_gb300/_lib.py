@@ -96,7 +96,6 @@ class Config(ctypes.Structure):
         ("exportdebugdata", ctypes.POINTER(ctypes.c_float)),
         ("errorcode", ctypes.c_int),
         ("errormsg", ctypes.c_char * 256),
-        ("complexpairs", ctypes.c_int),
     ]
 
 
@@ -109,7 +108,7 @@ class DevInfo(ctypes.Structure):
 
 # every symbol include/mcx_gb300.h declares
 EXPORTS = [
-    "mcx_initcfg", "mcx_clearcfg", "mcx_validatecfg", "mcx_list_gpu", "mcx_cleargpuinfo", "mcx_run_simulation",
+    "mcx_initcfg", "mcx_clearcfg", "mcx_validatecfg", "mcx_list_gpu", "mcx_cleargpuinfo", "mcx_run_simulation", "mcx_run_simulation_pairs",
     "mcx_normalize", "mcx_error", "mcx_last_error", "mcx_detreclen", "mcx_version", "mcx_rand_words", "mcx_rand_blocks", "mcx_config_sizeof",
     "mcx_config_offsetof", "mcx_release_sessions", "mcx_prepare_simulation",
     "mcxg_device_count", "mcxg_device_info", "mcxg_error_string", "mcxg_create", "mcxg_destroy",
@@ -144,6 +143,7 @@ def load():
     L.mcx_clearcfg.argtypes = [P(Config)]
     L.mcx_validatecfg.argtypes = [P(Config), vp, vp, ctypes.c_int]
     L.mcx_run_simulation.argtypes = [P(Config), vp, vp]
+    L.mcx_run_simulation_pairs.argtypes = [P(Config)]
     L.mcx_readconfig.argtypes = [ctypes.c_char_p, P(Config)]
     L.mcx_parsejson.argtypes = [ctypes.c_char_p, P(Config)]
     L.mcx_list_gpu.argtypes = [P(Config), P(ctypes.c_uint), P(P(GPUInfo))]

@@ -1453,7 +1453,7 @@ static void adjoint_jacobians(Config* cfg, mcxg_session* s, size_t nvox) {
 static __thread int prepare_only = 0;
 static __thread mcxg_session* prepared_session = NULL;
 
-static void run_simulation(Config* cfg) {
+static void run_simulation(Config* cfg, int pairs) {
     GPUInfo* gpu = NULL;
     /* temporaries live in thread-local slots so the library-mode error path
        (longjmp back to this frame) can free them */
@@ -1865,7 +1865,7 @@ static void run_simulation(Config* cfg) {
             device_check(mcxg_get_field_interleaved(s, dst, blockscale, nblocks), "reading the field");
         } else if (blockscale) {
             device_check(mcxg_get_field_blocks(s, dst, blockscale, nblocks), "reading the field");
-        } else if (cfg->complexpairs && cfg->omega > 0.f && !replay) {     /* never with shared photons */
+        } else if (pairs && cfg->omega > 0.f && !replay) {     /* never with shared photons */
             device_check(mcxg_get_field_pairs(s, dst, scale), "reading the field");
         } else {
             device_check(mcxg_get_field(s, dst, scale), "reading the field");
@@ -2154,17 +2154,25 @@ void mcx_keep_sessions(int keep) {
     pthread_mutex_unlock(&g_run_lock);
 }
 
-void mcx_run_simulation(Config* cfg, float* fluence, float* totalenergy) {
-    (void)fluence;
-    (void)totalenergy;
+static void run_locked(Config* cfg, int pairs) {
     pthread_mutex_lock(&g_run_lock);
     const int dev = mcxg_internal_current_device();
-    run_simulation(cfg);         /* library-mode errors return here through its own setjmp */
+    run_simulation(cfg, pairs);  /* library-mode errors return here through its own setjmp */
     if (!g_keep_sessions) {
         release_sessions();
     }
     mcxg_internal_restore_device(dev);
     pthread_mutex_unlock(&g_run_lock);
+}
+
+void mcx_run_simulation(Config* cfg, float* fluence, float* totalenergy) {
+    (void)fluence;
+    (void)totalenergy;
+    run_locked(cfg, 0);
+}
+
+void mcx_run_simulation_pairs(Config* cfg) {
+    run_locked(cfg, 1);
 }
 
 void mcx_run_batch(Config** cfgs, int n, unsigned int photons_per_thread, unsigned int flags) {
@@ -2193,7 +2201,7 @@ mcxg_session* mcx_prepare_simulation(Config* cfg) {
     pthread_mutex_lock(&g_run_lock);
     prepare_only = 1;
     prepared_session = NULL;
-    run_simulation(cfg);
+    run_simulation(cfg, 0);
     prepare_only = 0;
     mcxg_session* s = cfg->errorcode ? NULL : prepared_session;
     pthread_mutex_unlock(&g_run_lock);
@@ -2226,7 +2234,7 @@ static const struct {
     MCX_FIELD(failedlaunch), MCX_FIELD(threadused), MCX_FIELD(exportenergy), MCX_FIELD(savethreadenergy),
     MCX_FIELD(autotune), MCX_FIELD(savedetweight), MCX_FIELD(exportdetweight), MCX_FIELD(replaysiteown), MCX_FIELD(omega),
     MCX_FIELD(polprop), MCX_FIELD(polmedianum), {"lambda_", offsetof(Config, lambda)}, MCX_FIELD(srciquv),
-    MCX_FIELD(smatrix), MCX_FIELD(maxjumpdebug), MCX_FIELD(debugdatalen), MCX_FIELD(exportdebugdata), MCX_FIELD(errorcode), MCX_FIELD(errormsg), MCX_FIELD(complexpairs),
+    MCX_FIELD(smatrix), MCX_FIELD(maxjumpdebug), MCX_FIELD(debugdatalen), MCX_FIELD(exportdebugdata), MCX_FIELD(errorcode), MCX_FIELD(errormsg),
 };
 
 size_t mcx_config_sizeof(void) {

@@ -353,8 +353,7 @@ def run(cfg=None, **kwargs):
         else:
             L.mcx_validatecfg(ctypes.byref(C), None, None, 0)
         _check(C)
-        C.complexpairs = 1
-        L.mcx_run_simulation(ctypes.byref(C), None, None)
+        L.mcx_run_simulation_pairs(ctypes.byref(C))
         _check(C)
         return _outputs(cfg, C)
     finally:
@@ -450,7 +449,7 @@ def _outputs(cfg, C):
         n = C.dim.x * C.dim.y * C.dim.z * gates * nsrc * ndetblk * nshare
         f = _take(C, "exportfield", ctypes.c_float, n * comps)
         if rffwd:
-            # {real, imaginary} pairs from the device (C.complexpairs): complex64 as they lie
+            # {real, imaginary} pairs from the device (mcx_run_simulation_pairs): complex64 as they lie
             # (50 gates of 216,000 voxels: 25 ms to build from two planes)
             f = f.view(np.complex64)
         if rfrep:
