@@ -265,24 +265,19 @@ __device__ __forceinline__ double merged_at(const float* __restrict__ f, size_t 
 /* (count x unit + remainder) x scale rounded to float, the same bits as
    cell_value() * scale, with the FP64 pipe (two operations a cycle and SM)
    left to what needs it: nothing for an untouched element, and without a
-   remainder one product, unit being a power of two.  plain: 0 x scale is +0; a
-   run that launched no weight has an infinite factor and NaN everywhere. */
-__device__ __forceinline__ float merged_f32(long long k, float r, double unit, double scale, bool plain) {
+   remainder one product, unit being a power of two. */
+__device__ __forceinline__ float merged_f32(long long k, float r, double unit, double scale) {
     if (r != 0.f) {
         return (float)(((double)k * unit + (double)r) * scale);
     }
-    return (k || !plain) ? (float)((double)k * (unit * scale)) : 0.f;
-}
-
-bool plain_scales(const double* scales, size_t n) {
-    return std::all_of(scales, scales + n, [](double v) { return std::isfinite(v) && !std::signbit(v); });
+    return k ? (float)((double)k * (unit * scale)) : 0.f;
 }
 
 /* out[i] = merged_f32() of the elements [0, n) from `first` on, scaled by
    scale(i): four elements' loads in flight a thread */
 template <class Scale>
 __device__ __forceinline__ void merge_range(const float* __restrict__ f, size_t total, size_t first, size_t n, double unit,
-                                            Scale scale, bool plain, float* __restrict__ out) {
+                                            Scale scale, float* __restrict__ out) {
     const long long* hi = reinterpret_cast<const long long*>(f) + first;
     const float* lo = f + 2 * total + first;
     const size_t stride = (size_t)gridDim.x * blockDim.x;
@@ -299,21 +294,19 @@ __device__ __forceinline__ void merge_range(const float* __restrict__ f, size_t 
         for (int u = 0; u < 4; u++) {
             const size_t j = i + u * stride;
             if (j < n) {
-                out[first + j] = ((k[u] | (long long)__float_as_uint(r[u])) || !plain) ? merged_f32(k[u], r[u], unit, scale(j), plain)
-                                                                                      : 0.f;
+                out[first + j] = (k[u] | (long long)__float_as_uint(r[u])) ? merged_f32(k[u], r[u], unit, scale(j)) : 0.f;
             }
         }
     }
 }
 
-__global__ void field_merge_f32(const float* __restrict__ f, size_t total, double unit, double scale, bool plain,
+__global__ void field_merge_f32(const float* __restrict__ f, size_t total, double unit, double scale,
                                 float* __restrict__ out) {
-    merge_range(f, total, 0, total, unit, [=](size_t) { return scale; }, plain, out);
+    merge_range(f, total, 0, total, unit, [=](size_t) { return scale; }, out);
 }
 
 /* a complex field's two components as pairs */
-__global__ void field_merge_pairs(const float* __restrict__ f, size_t n, double unit, double scale, bool plain,
-                                  float2* __restrict__ out) {
+__global__ void field_merge_pairs(const float* __restrict__ f, size_t n, double unit, double scale, float2* __restrict__ out) {
     const long long* hi = reinterpret_cast<const long long*>(f);
     const float* lo = f + 4 * n;
     const size_t stride = (size_t)gridDim.x * blockDim.x;
@@ -330,7 +323,7 @@ __global__ void field_merge_pairs(const float* __restrict__ f, size_t n, double 
         for (int u = 0; u < 4; u += 2) {
             const size_t j = i + (u >> 1) * stride;
             if (j < n) {
-                out[j] = make_float2(merged_f32(k[u], r[u], unit, scale, plain), merged_f32(k[u + 1], r[u + 1], unit, scale, plain));
+                out[j] = make_float2(merged_f32(k[u], r[u], unit, scale), merged_f32(k[u + 1], r[u + 1], unit, scale));
             }
         }
     }
@@ -348,8 +341,8 @@ __global__ void field_merge_interleaved(const float* __restrict__ f, size_t n, s
 }
 
 __global__ void field_merge_blocks(const float* __restrict__ f, size_t n, size_t total, double unit, size_t blocklen,
-                                   const double* __restrict__ scales, bool plain, float* __restrict__ out) {
-    merge_range(f, total, 0, total, unit, [=](size_t i) { return scales[(i % n) / blocklen]; }, plain, out);
+                                   const double* __restrict__ scales, float* __restrict__ out) {
+    merge_range(f, total, 0, total, unit, [=](size_t i) { return scales[(i % n) / blocklen]; }, out);
 }
 
 /* reciprocals of each simulation's property rows, as the single-simulation
@@ -421,12 +414,12 @@ __global__ void __launch_bounds__(256) batch_energy_final(const double* __restri
 
 /* merged, scaled field of every simulation: row y of the grid is simulation y */
 __global__ void batch_merge(const float* __restrict__ f, unsigned long long total, const mcxg_simdesc* __restrict__ sims,
-                            const double* __restrict__ scales, bool plain, float* __restrict__ out) {
+                            const double* __restrict__ scales, float* __restrict__ out) {
     const mcxg_simdesc& d = sims[blockIdx.y];
     const unsigned long long off = d.field_off;
     const unsigned int n = d.kp.fieldlen;
     const double sc = scales[blockIdx.y];
-    merge_range(f, total, off, n, (double)d.kp.fxunit, [=](size_t) { return sc; }, plain, out);
+    merge_range(f, total, off, n, (double)d.kp.fxunit, [=](size_t) { return sc; }, out);
 }
 
 /* every simulation's compensated field merged in FP64, unscaled */
@@ -1812,8 +1805,7 @@ int mcxg_get_field(mcxg_session* s, float* out, double scale) {
     if (rc) {
         return rc;
     }
-    field_merge_f32<<<grid_for(s, total), 256, 0, s->st>>>(s->d_field, total, (double)s->kp.fxunit, scale,
-                                                           plain_scales(&scale, 1), (float*)s->d_out);
+    field_merge_f32<<<grid_for(s, total), 256, 0, s->st>>>(s->d_field, total, (double)s->kp.fxunit, scale, (float*)s->d_out);
     s->out_valid = true;
     MCXG_TRY(cudaMemcpyAsync(out, s->d_out, sizeof(float) * total, cudaMemcpyDeviceToHost, s->st));
     MCXG_TRY(cudaStreamSynchronize(s->st));
@@ -1830,8 +1822,7 @@ int mcxg_get_field_pairs(mcxg_session* s, float* out, double scale) {
     if (rc) {
         return rc;
     }
-    field_merge_pairs<<<grid_for(s, n), 256, 0, s->st>>>(s->d_field, n, (double)s->kp.fxunit, scale, plain_scales(&scale, 1),
-                                                         (float2*)s->d_out);
+    field_merge_pairs<<<grid_for(s, n), 256, 0, s->st>>>(s->d_field, n, (double)s->kp.fxunit, scale, (float2*)s->d_out);
     s->out_valid = false;
     MCXG_TRY(cudaGetLastError());
     MCXG_TRY(cudaMemcpyAsync(out, s->d_out, sizeof(float) * 2 * n, cudaMemcpyDeviceToHost, s->st));
@@ -1854,7 +1845,7 @@ int mcxg_get_field_blocks(mcxg_session* s, float* out, const double* scales, uin
     }
     MCXG_TRY(cudaMemcpyAsync(s->d_scales, scales, sizeof(double) * nblocks, cudaMemcpyHostToDevice, s->st));
     field_merge_blocks<<<grid_for(s, total), 256, 0, s->st>>>(s->d_field, n, total, (double)s->kp.fxunit, n / nblocks,
-                                                              s->d_scales, plain_scales(scales, nblocks),
+                                                              s->d_scales,
                                                               (float*)s->d_out);
     s->out_valid = true;
     MCXG_TRY(cudaMemcpyAsync(out, s->d_out, sizeof(float) * total, cudaMemcpyDeviceToHost, s->st));
@@ -2459,8 +2450,7 @@ int mcxg_batch_get_field(mcxg_session* s, float* out, const double* scales) {
     }
     MCXG_TRY(cudaMemcpyAsync(s->d_scales, scales, sizeof(double) * s->nsim, cudaMemcpyHostToDevice, s->st));
     MCXG_TRY(cudaMemsetAsync(s->d_bout, 0, sizeof(float) * (size_t)s->totalfield, s->st));
-    batch_merge<<<dim3(64, s->nsim), 256, 0, s->st>>>(s->d_bfield, s->totalfield, s->d_sims, s->d_scales,
-                                                      plain_scales(scales, s->nsim), s->d_bout);
+    batch_merge<<<dim3(64, s->nsim), 256, 0, s->st>>>(s->d_bfield, s->totalfield, s->d_sims, s->d_scales, s->d_bout);
     MCXG_TRY(cudaMemcpyAsync(out, s->d_bout, sizeof(float) * (size_t)s->totalfield, cudaMemcpyDeviceToHost, s->st));
     MCXG_TRY(cudaStreamSynchronize(s->st));
     MCXG_TRY(cudaGetLastError());

@@ -70,49 +70,3 @@ def test_both_gradient_passes_on_one_kernel():
             assert _usual(g.L, g.s) == 0
     finally:
         g.close()
-
-
-@pytest.mark.parametrize("scale", [np.inf, np.nan, -np.inf, -2.0, 0.0, 3.0])
-@pytest.mark.parametrize("omega", [0, 2 * np.pi * 1e8])
-def test_untouched_elements_take_the_scale(scale, omega):
-    """An element that no photon touched is 0 x scale: NaN under an infinite factor, as in a run that launched nothing."""
-    from mcxcl_gb300 import _lib, pmcxcl
-    L, C = _lib.load(), _lib.Config()
-    try:
-        pmcxcl.parse_config(cases.small_two_media(nphoton=300, omega=omega), C)
-        L.mcx_validatecfg(ctypes.byref(C), None, None, 0)
-        s = L.mcx_prepare_simulation(ctypes.byref(C))
-        pmcxcl._check(C)
-        assert L.mcxg_simulate(s, 2, ctypes.byref(ctypes.c_float())) == 0
-        n = 40 ** 3 * 20
-        raw, got = np.zeros((2, n), np.float32), np.zeros((2, n), np.float32)
-        comps = 2 if omega else 1
-        assert L.mcxg_get_field(s, raw.ctypes.data, 1.0) == 0 and L.mcxg_get_field(s, got.ctypes.data, scale) == 0
-        with np.errstate(invalid="ignore"):
-            want = (raw.astype(np.float64) * scale).astype(np.float32)
-        assert (raw[:comps] == 0).mean() > 0.5 and (raw[:comps] != 0).any()
-        # raw is rounded to float before the product here, and after it there
-        assert np.allclose(got[:comps], want[:comps], rtol=2.5e-7, atol=0, equal_nan=True)
-        if omega:
-            pairs = np.zeros((n, 2), np.float32)
-            assert L.mcxg_get_field_pairs(s, pairs.ctypes.data, scale) == 0
-            assert np.array_equal(pairs.T, got, equal_nan=True)
-        else:
-            blocks, scales = np.zeros(n, np.float32), np.array([scale, 1.0] * 10)
-            assert L.mcxg_get_field_blocks(ctypes.c_void_p(s), ctypes.c_void_p(blocks.ctypes.data),
-                                           ctypes.c_void_p(scales.ctypes.data), ctypes.c_uint32(20)) == 0
-            both = blocks.reshape(10, 2, -1)
-            assert np.array_equal(both[:, 0], got[0].reshape(10, 2, -1)[:, 0], equal_nan=True)
-            assert np.array_equal(both[:, 1], raw[0].reshape(10, 2, -1)[:, 1])
-    finally:
-        L.mcx_clearcfg(ctypes.byref(C))
-
-
-def test_a_run_that_launches_nothing():
-    import mcxcl_gb300
-    cfg = cases.small_two_media(nphoton=300, maxvoidstep=1, issavedet=0, issaveseed=0)
-    cfg.pop("detpos")
-    r = mcxcl_gb300.run(cfg)
-    assert r["stat"]["energytot"] == 0 and np.isnan(r["flux"]).all()
-    many = mcxcl_gb300.run_batch([cfg, dict(cfg, maxvoidstep=1000)])
-    assert np.isnan(many[0]["flux"]).all() and np.isfinite(many[1]["flux"]).all() and many[1]["flux"].max() > 0
