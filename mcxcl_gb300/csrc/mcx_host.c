@@ -1610,6 +1610,14 @@ static void run_simulation(Config* cfg, int pairs) {
         kp.oddphoton = (int)((float)cfg->nphoton * workload0 / (fullload * (float)cfg->respin) -
                              (float)((size_t)kp.threadphoton * autothread));
         device_check(mcxg_set_params(s, &kp, sizeof(kp)), "updating parameters");
+        if (iter == 0) {
+            /* a cached session keeps neither the last run's launch shape nor its trajectory
+               records, whether this call runs the problem or only prepares it */
+            device_check(mcxg_set_launch(s, 0, 0), "resetting the launch shape");
+            /* MCX_DEBUG_MOVE (2) and MCX_DEBUG_MOVE_ONLY (8) both record (mcx_host.cpp:702, 1173) */
+            device_check(mcxg_set_trajectory(s, (cfg->debuglevel & 10) ? cfg->maxjumpdebug : 0u),
+                         "allocating the trajectory records");
+        }
         if (prepare_only) {
             /* mcx_prepare_simulation: everything is resident, nothing has run */
             prepared_session = s;
@@ -1618,13 +1626,6 @@ static void run_simulation(Config* cfg, int pairs) {
         }
         unsigned int flags = (cfg->exactmath ? MCXG_EXACT : 0u) | (iter ? MCXG_KEEP : 0u) |
                              ((cfg->debuglevel & 1) ? MCXG_RNGDUMP : 0u);
-        if (iter == 0) {
-            device_check(mcxg_set_launch(s, 0, 0), "resetting the launch shape");
-            /* MCX_DEBUG_MOVE (2) and MCX_DEBUG_MOVE_ONLY (8) both record (mcx_host.cpp:702, 1173);
-               set before any launch so a cached session never keeps the last run's setting */
-            device_check(mcxg_set_trajectory(s, (cfg->debuglevel & 10) ? cfg->maxjumpdebug : 0u),
-                         "allocating the trajectory records");
-        }
         /* trajectory runs take the general instantiation and record at every
            launch: they are not tuned (the tuned shape is for the common one) */
         if (cfg->autotune && !cfg->exactmath && !(cfg->debuglevel & 11)) {
@@ -2038,6 +2039,7 @@ static void batch_run(Config** cfgs, int n, unsigned int photons_per_thread, uns
     if (!s) {
         MCX_ERROR(-99, "failed to open a CUDA session on the selected GPU");
     }
+    device_check(mcxg_set_launch(s, 0, 0), "resetting the launch shape");
     device_check(mcxg_batch_set_words(s, bdesc, sizeof(mcxg_simdesc), (uint32_t)n, bwords, nmedia), "uploading the batch");
     float kms = 0.f;
     device_check(mcxg_batch_simulate(s, flags | (relerr ? MCXG_VERIFY : 0u), &kms), "running the batch");

@@ -70,3 +70,40 @@ def test_both_gradient_passes_on_one_kernel():
             assert _usual(g.L, g.s) == 0
     finally:
         g.close()
+
+
+def _launch(L, s):
+    grid, block = ctypes.c_int(), ctypes.c_int()
+    assert L.mcxg_get_launch(s, ctypes.byref(grid), ctypes.byref(block), None) == 0
+    return grid.value, block.value
+
+
+def _plain(**kw):
+    cfg = cases.small_two_media(**dict(dict(issavedet=0, issaveseed=0), **kw))
+    cfg.pop("detpos")
+    return cfg
+
+
+def test_a_tuned_shape_ends_with_its_run():
+    """The shape that a small tuned run chose is not the next batch's or gradient's."""
+    import mcxcl_gb300
+    from mcxcl_gb300 import diff
+    L, s = _session()
+    sims = [_plain(nphoton=20000, seed=k + 1) for k in range(4)]
+    mcxcl_gb300.run_batch(sims)
+    batch = _launch(L, s), _usual(L, s)
+    assert batch[1] == 1
+    cfg, shapes = _plain(nphoton=2000000), []
+    for before in ({}, dict(nphoton=50000, autotune=1), dict(nphoton=50000, autotune=1, gscatter=1 << 24), dict(nphoton=300, debuglevel="M")):
+        mcxcl_gb300.run(_plain(**before))
+        g = diff.FluenceGradient(cfg)
+        try:
+            f = g.forward()
+            shapes.append((_launch(L, s), _usual(L, s)))
+            g.backward(np.ones(f.shape))
+        finally:
+            g.close()
+        mcxcl_gb300.run(_plain(**before))
+        mcxcl_gb300.run_batch(sims)
+        assert (_launch(L, s), _usual(L, s)) == batch
+    assert shapes == [shapes[0]] * 4 and shapes[0][1] == 1
