@@ -591,8 +591,9 @@ int  mcxg_energy_sum_noalloc(int device, const float* d_energy, uint32_t nthread
 /* The persistent grid actually used by the last launch. */
 int  mcxg_get_launch(mcxg_session* s, int* grid, int* block, int* regs);
 /* Which transport kernel the last mcxg_simulate or mcxg_batch_simulate ran: 1
-   the usual configurations' (mcx_kernel_label.cuh), 0 the general one. */
-int  mcxg_get_kernel(mcxg_session* s, int* usual);
+   the usual configurations' (mcx_kernel_label.cuh), 0 the general one; and how
+   many lanes of each warp took work (32 but in runs of few photons). */
+int  mcxg_get_kernel(mcxg_session* s, int* usual, int* lanes);
 
 #ifdef __cplusplus
 }

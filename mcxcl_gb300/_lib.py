@@ -195,7 +195,7 @@ def load():
     L.mcxg_get_detected.argtypes = [vp, vp, vp, P(ctypes.c_uint32)]
     L.mcxg_get_counters.argtypes = [vp, vp, vp]
     L.mcxg_get_launch.argtypes = [vp, P(ctypes.c_int), P(ctypes.c_int), P(ctypes.c_int)]
-    L.mcxg_get_kernel.argtypes = [vp, P(ctypes.c_int)]
+    L.mcxg_get_kernel.argtypes = [vp, P(ctypes.c_int), P(ctypes.c_int)]
     L.mcxg_fp32_peak.argtypes = [vp, P(ctypes.c_double)]
     L.mcxg_energy_sum_noalloc.argtypes = [ctypes.c_int, vp, ctypes.c_uint32, vp]
     L.mcxg_autotune.argtypes = [vp, ctypes.c_uint32, P(ctypes.c_int), P(ctypes.c_int), P(ctypes.c_int)]

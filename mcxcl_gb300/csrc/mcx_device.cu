@@ -144,7 +144,7 @@ struct mcxg_session {
     mcxg::KArgs::Tile tile_used{};   /* the last launch's tile (nx = 0: none) */
     int tuned = 0;                   /* 1 once mcxg_autotune picked a shape for this problem */
     int tuned_noagg = 0;
-    int grid = 0, block = 0, regs = 0, usual = 0;
+    int grid = 0, block = 0, regs = 0, usual = 0, lanes = 32;
 };
 
 namespace {
@@ -564,7 +564,7 @@ size_t shared_bytes(const mcxg_kparams& kp, int block) {
     return (size_t)kp.medianum * 32 + (size_t)block * 32 + (size_t)(kp.nphase + kp.nangle) * 4 + det * (size_t)block * 4;
 }
 
-/* Blocks per SM (of 256 threads) and lanes per warp for a run of `photons`.
+/* Blocks per SM (of 256 threads) for a run of `photons`, and lanes per warp.
    A photon takes up to thousands of steps one after another, so a run cannot
    end before its longest photon, and a step takes the longer the more warps
    share the SM (cube: 3 us at 32 warps, 0.55 us at a few) and the more lanes
@@ -579,18 +579,20 @@ size_t shared_bytes(const mcxg_kparams& kp, int block) {
    step, gain from fewer warps only below 1,000 photons an SM (the replay of
    9,000 photons 4.7 -> 3.7 ms); at 1e6 photons 2 blocks were 5 to 10 % slower
    than 4. */
-void shape_for(unsigned long long photons, int sms, bool label, int* blocks, unsigned int* lanes) {
+int blocks_for(unsigned long long photons, int sms, bool label) {
     const unsigned long long q = photons / (unsigned int)sms;
-    *lanes = 32u;
-    if (q <= 96) {
-        *blocks = 2;
-        *lanes = std::max(1u, (unsigned int)(q + 15) / 16);       /* one photon a lane, over 16 warps */
-    } else if (q <= 1000) {
-        *blocks = 1;
-        *lanes = std::min(32u, (unsigned int)(q + 7) / 8);
-    } else {
-        *blocks = !label ? 4 : (q <= 10000 ? 2 : (q <= 35000 ? 3 : 4));
+    if (q <= 1000) {
+        return q <= 96 ? 2 : 1;
     }
+    return !label ? 4 : (q <= 10000 ? 2 : (q <= 35000 ? 3 : 4));
+}
+
+/* Lanes of each warp that take work: one photon a lane as long as the warps
+   that are resident have a lane for each.  Asked once the blocks are known, a
+   caller's own and what shared memory leaves of them included. */
+unsigned int lanes_for(unsigned long long photons, int sms, int warps) {
+    const unsigned long long q = photons / (unsigned int)sms;
+    return (unsigned int)std::min(32ull, std::max(1ull, (q + warps - 1) / warps));
 }
 
 /* What mcx_transport_label does for a run (RUN_FWD ..), or -1: it takes 3-D
@@ -631,6 +633,23 @@ int label_run(const mcxg_kparams& kp) {
 size_t label_shared_bytes(const mcxg_kparams& kp) {
     const size_t kinds = kp.savedet && kp.maxmedia ? kp.partialdata / kp.maxmedia : 0;
     return (size_t)mcxg::kLabelBlock * 32 + (size_t)kp.medianum * 48 + kinds * kp.medianum * mcxg::kLabelBlock * 4 + (size_t)kp.nangle * 4;
+}
+
+/* What the usual configurations' kernel does for this problem on this session,
+   in blocks of `block` threads with plain deposits, or -1 where the general
+   kernel runs it.  The gradient's passes stay on the general kernel.  The
+   second one's float sums drop up to 1e-4 of the hottest voxels' gradients, how
+   much depends on the order of the additions; the first one's totals are the same
+   to the bit on either kernel, but with another kernel before it the second pass
+   starts out of step and its order varies more (two calls' dL/dmus 5.7e-6 apart
+   on average, 3.7 to 4.1e-6 with its own kernel before it; 1e6 photons, 60^3). */
+int usual_run(const mcxg_session* s, const mcxg_kparams& kp, unsigned int flags, int block) {
+    if ((flags & (MCXG_EXACT | MCXG_RNGDUMP | MCXG_GENERAL | MCXG_VERIFY | MCXG_ADJ1 | MCXG_ADJ2)) || s->npol || s->maxjump ||
+            block != mcxg::kLabelBlock) {
+        return -1;
+    }
+    /* a slot more for each kind of record: the last media that fit the other kernel's layout */
+    return label_shared_bytes(kp) > s->info.sharedmem_per_block ? -1 : label_run(kp);
 }
 
 /* q = umulhi(n, m) >> sh equals n / d for every n < bound: m = ceil(2^(32+sh) / d)
@@ -1601,17 +1620,7 @@ int mcxg_simulate(mcxg_session* s, unsigned int flags, float* kernel_ms) {
         }
     }
     /* the usual configurations have a kernel of their own */
-    /* The gradient's passes stay on the general kernel.  The second one's float
-       sums drop up to 1e-4 of the hottest voxels' gradients, how much depends on
-       the order of the additions; the first one's totals are the same to the bit on
-       either kernel, but with another kernel before it the second pass starts out
-       of step and its order varies more (two calls' dL/dmus 5.7e-6 apart on
-       average, 3.7 to 4.1e-6 with its own kernel before it; 1e6 photons, 60^3) */
-    int lrun = (exact || pol || svmc || xmedia || s->maxjump || adjmode || (flags & MCXG_GENERAL) || block != mcxg::kLabelBlock ||
-                      (lflags & (mcxg::LF_WAGG | mcxg::LF_TILE | mcxg::LF_ACC64))) ? -1 : label_run(kp);
-    if (lrun >= 0 && label_shared_bytes(kp) > s->info.sharedmem_per_block) {
-        lrun = -1;         /* a slot more for each kind of record: the last media that fit the other kernel's layout */
-    }
+    const int lrun = (lflags & (mcxg::LF_WAGG | mcxg::LF_TILE)) ? -1 : usual_run(s, kp, flags, block);
     const bool label = lrun >= 0;
     s->usual = label;
     if (label) {
@@ -1631,12 +1640,9 @@ int mcxg_simulate(mcxg_session* s, unsigned int flags, float* kernel_ms) {
         return MCXG_ERR_LIMIT;
     }
     int bpsm = exact ? 2 : bpsm_sel;
-    a.lanes = 32;
+    const unsigned long long photons = (unsigned long long)kp.threadphoton * kp.nthread + (unsigned long long)std::max(kp.oddphoton, 0);
     if (!exact && adjmode != 2u && !s->block_req && !s->bpsm_req) {
-        int few = 0;
-        shape_for((unsigned long long)kp.threadphoton * kp.nthread + (unsigned long long)std::max(kp.oddphoton, 0),
-                  s->info.sm, label, &few, &a.lanes);
-        bpsm = std::min(bpsm, few);
+        bpsm = std::min(bpsm, blocks_for(photons, s->info.sm, label));
     }
     if (!exact) {
         /* never more blocks than fit at once: a persistent grid must be resident */
@@ -1649,6 +1655,8 @@ int mcxg_simulate(mcxg_session* s, unsigned int flags, float* kernel_ms) {
     if (bpsm < 1) {
         bpsm = 1;
     }
+    a.lanes = (exact || adjmode == 2u) ? 32u : lanes_for(photons, s->info.sm, bpsm * block / 32);
+    s->lanes = (int)a.lanes;
     int grid = s->info.sm * bpsm;
     s->grid = grid;
     s->block = block;
@@ -1706,14 +1714,12 @@ int mcxg_autotune(mcxg_session* s, uint32_t sample_photons, int* block, int* blo
         int block, bpsm, noagg;
     } cands[] = {{256, 4, 1}, {128, 8, 1}, {64, 16, 1}, {256, 2, 1}, {128, 4, 1}, {0, 0, 0}};
     const int ncand = (int)(sizeof(cands) / sizeof(cands[0]));
-    /* the usual configurations' kernel runs blocks of 256 in one register
-       budget; how many a SM follows from the whole run's photons (shape_for), as
-       a sample, mostly tail, always favours few */
-    const bool label = label_run(full) >= 0 && !s->npol && !s->maxjump;
-    if (label) {
-        unsigned int lanes = 32;
-        shape_for(total, s->info.sm, true, &cands[0].bpsm, &lanes);
-    }
+    /* how many blocks of 256 a SM follows from the whole run's photons
+       (blocks_for), as a sample, mostly tail, always favours few; the usual
+       configurations' kernel has no other shape of 256 threads, its blocks having
+       one register budget */
+    const bool label = !s->tile_req && usual_run(s, full, 0u, mcxg::kLabelBlock) >= 0;
+    cands[0].bpsm = blocks_for(total, s->info.sm, label);
     float best = 1e30f;
     Cand pick = cands[0];
     int keep_block = s->block_req, keep_bpsm = s->bpsm_req;
@@ -2376,6 +2382,7 @@ int mcxg_batch_simulate(mcxg_session* s, unsigned int flags, float* kernel_ms) {
         lflags |= mcxg::LF_LABEL;
     }
     s->usual = (lflags & mcxg::LF_LABEL) != 0;
+    s->lanes = 32;
     int occ = 0;
     MCXG_TRY(mcxg::batch_occupancy(lflags, block, std::min<uint32_t>(s->nsim, mcxg::kBatchWave), &occ));
     int bpsm = std::max(1, std::min(bpsm_req, occ > 0 ? occ : bpsm_req));
@@ -2530,11 +2537,16 @@ int mcxg_get_launch(mcxg_session* s, int* grid, int* block, int* regs) {
     return MCXG_OK;
 }
 
-int mcxg_get_kernel(mcxg_session* s, int* usual) {
-    if (!s || !usual) {
+int mcxg_get_kernel(mcxg_session* s, int* usual, int* lanes) {
+    if (!s) {
         return MCXG_ERR_ARG;
     }
-    *usual = s->usual;
+    if (usual) {
+        *usual = s->usual;
+    }
+    if (lanes) {
+        *lanes = s->lanes;
+    }
     return MCXG_OK;
 }
 

@@ -1026,7 +1026,8 @@ static uint64_t mix64(uint64_t h, uint64_t v) {
 }
 
 /* what the launch shape depends on: the volume, the media, the source, the
-   outputs compiled in and the photon budget per thread */
+   outputs compiled in, the photon budget per thread and what decides between
+   the two transport kernels (label_run in mcx_device.cu) */
 static uint64_t tune_signature(const Config* cfg, const mcxg_kparams* kp) {
     uint64_t h = 1469598103934665603ull;
     h = mix64(h, kp->nvox);
@@ -1034,6 +1035,11 @@ static uint64_t tune_signature(const Config* cfg, const mcxg_kparams* kp) {
     h = mix64(h, kp->fieldlen);
     h = mix64(h, (uint64_t)kp->medianum << 32 | (uint32_t)kp->srctype);
     h = mix64(h, (uint64_t)kp->savedet << 8 | (uint64_t)kp->dorefl_compiled << 4 | (uint64_t)kp->issaveref);
+    h = mix64(h, (uint64_t)kp->mediaformat << 32 | (uint64_t)kp->mediaword << 16 | (uint64_t)kp->outputtype << 8 |
+                 (uint64_t)(kp->omega > 0.f) << 4 | (uint64_t)kp->replay << 3 | (uint64_t)kp->save2pt << 2 | kp->is2d);
+    h = mix64(h, (uint64_t)kp->nphase << 32 | kp->gscatter);
+    h = mix64(h, (uint64_t)kp->srcnum << 32 | (uint64_t)kp->extrasrclen << 16 | kp->savedetflag);
+    h = mix64(h, (uint64_t)kp->nangle << 32 | cfg->polmedianum);
     h = mix64(h, kp->nthread);
     h = mix64(h, (uint64_t)(cfg->nphoton / 1000));
     h = mix64(h, (uint64_t)cfg->dim.y << 32 | cfg->dim.z);

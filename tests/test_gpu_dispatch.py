@@ -25,9 +25,13 @@ def _session():
 
 
 def _usual(L, s):
-    usual = ctypes.c_int(-1)
-    assert L.mcxg_get_kernel(s, ctypes.byref(usual)) == 0
-    return usual.value
+    return _kernel(L, s)[0]
+
+
+def _kernel(L, s):
+    usual, lanes = ctypes.c_int(-1), ctypes.c_int(-1)
+    assert L.mcxg_get_kernel(s, ctypes.byref(usual), ctypes.byref(lanes)) == 0
+    return usual.value, lanes.value
 
 
 @pytest.mark.parametrize("name", list(CASES))
@@ -107,3 +111,56 @@ def test_a_tuned_shape_ends_with_its_run():
         mcxcl_gb300.run_batch(sims)
         assert (_launch(L, s), _usual(L, s)) == batch
     assert shapes == [shapes[0]] * 4 and shapes[0][1] == 1
+
+
+def test_tuned_runs_of_few_photons_spread_their_lanes():
+    import mcxcl_gb300
+    L, s = _session()
+    mcxcl_gb300.run(_plain(nphoton=10000))
+    assert _kernel(L, s)[0] == 1 and _kernel(L, s)[1] < 32
+    mcxcl_gb300.run(_plain(nphoton=10000, autotune=1))
+    grid, block = _launch(L, s)
+    sms = mcxcl_gb300.gpuinfo()[0]["sm"]
+    warps = grid // sms * block // 32
+    assert _kernel(L, s)[1] == min(32, -(-(10000 // sms) // warps)) < 32
+
+
+def test_the_kernels_are_tuned_apart():
+    """A general run's tuned shape is not taken for the same problem on the usual configurations' kernel."""
+    import mcxcl_gb300
+    L, s = _session()
+    sms = mcxcl_gb300.gpuinfo()[0]["sm"]
+    cfg = _plain(nphoton=20000 * sms, autotune=1)
+    mcxcl_gb300.run(dict(cfg, gscatter=1 << 24))
+    assert _usual(L, s) == 0
+    mcxcl_gb300.run(cfg)
+    assert _usual(L, s) == 1 and _launch(L, s) == (3 * sms, 256)
+
+
+@pytest.mark.parametrize("general", [0, 1 << 24])
+@pytest.mark.parametrize("photons", [200, 20000, 200000])
+def test_every_shape_runs_every_photon(general, photons):
+    """Shapes of few warps and lanes, the caller's own included: the same energies as the automatic one."""
+    from mcxcl_gb300 import _lib, pmcxcl
+    L, C, got = _lib.load(), _lib.Config(), []
+    try:
+        pmcxcl.parse_config(dict(_plain(nphoton=photons), **({"gscatter": general} if general else {})), C)
+        L.mcx_validatecfg(ctypes.byref(C), None, None, 0)
+        s = L.mcx_prepare_simulation(ctypes.byref(C))
+        pmcxcl._check(C)
+        for shape in ((0, 0), (256, 1), (256, 3), (256, 4), (128, 2), (32, 1), (64, 16)):
+            for flags in (2, 16):                                        # plain and aggregated deposits
+                assert L.mcxg_set_launch(s, *shape) == 0
+                assert L.mcxg_simulate(s, flags, ctypes.byref(ctypes.c_float())) == 0
+                esc, tot = ctypes.c_double(), ctypes.c_double()
+                assert L.mcxg_get_energy(s, ctypes.byref(esc), ctypes.byref(tot)) == 0
+                field = np.zeros(40 ** 3 * 20)
+                assert L.mcxg_get_field_f64(s, field.ctypes.data) == 0
+                got.append((_usual(L, s), tot.value, esc.value, field.sum()))
+        assert L.mcxg_set_launch(s, 0, 0) == 0
+    finally:
+        L.mcx_clearcfg(ctypes.byref(C))
+    assert len({g[0] for g in got}) == (1 if general else 2)
+    for g in got:
+        # the instantiations of the general kernel contract differently: a path may part from another's
+        assert g[1] == photons and abs(g[2] - got[0][2]) <= 2e-3 * photons ** 0.5 * 10 and abs(g[3] / got[0][3] - 1) <= 0.02
