@@ -68,15 +68,11 @@ cudaError_t batch_launch(const KArgs& a, int flags, int grid, int block, cudaStr
     return cudaLaunchKernel(select(flags), dim3(grid), dim3(block), args, batch_shared_bytes(flags, block, a.nsim), st);
 }
 
-/* resident blocks a SM; also admits the shared memory of a wave of nsim */
+/* resident blocks a SM */
 cudaError_t batch_occupancy(int flags, int block, unsigned int nsim, int* blocks_per_sm) {
+    static_assert(LB_BLOCK * sizeof(ColdState) + kBatchWave * LabelPS<VOL_LABEL, DET_NONE>::kSim * sizeof(float4) <= 48 * 1024,
+                  "a whole wave fits the shared memory that needs no asking for");
     const size_t smem = batch_shared_bytes(flags, block, nsim);
-    if (smem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(select(flags), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) {
-            return e;
-        }
-    }
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, select(flags), block, smem);
 }
 

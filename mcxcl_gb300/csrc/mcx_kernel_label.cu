@@ -64,20 +64,22 @@ static void* select(int flags) {
     return (flags & LF_MUA) ? kvol<VOL_MUA>(flags) : kvol<VOL_LABEL>(flags);
 }
 
+/* more than 48 KB of shared memory a block has to be asked for, before the occupancy as before the launch */
+static cudaError_t admit(const void* f, size_t smem) {
+    return smem > 48 * 1024 ? cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) : cudaSuccess;
+}
+
 cudaError_t label_launch(const KArgs& a, int flags, int grid, int block, size_t smem, cudaStream_t st) {
     void* f = select(flags);
-    if (smem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) {
-            return e;
-        }
-    }
+    const cudaError_t e = admit(f, smem);
     void* args[] = {(void*)&a};
-    return cudaLaunchKernel(f, dim3(grid), dim3(block), args, smem, st);
+    return e == cudaSuccess ? cudaLaunchKernel(f, dim3(grid), dim3(block), args, smem, st) : e;
 }
 
 cudaError_t label_occupancy(int flags, int block, size_t smem, int* blocks_per_sm) {
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, select(flags), block, smem);
+    void* f = select(flags);
+    const cudaError_t e = admit(f, smem);
+    return e == cudaSuccess ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, f, block, smem) : e;
 }
 
 cudaError_t label_attributes(int flags, cudaFuncAttributes* attr) {

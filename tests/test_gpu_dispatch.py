@@ -164,3 +164,38 @@ def test_every_shape_runs_every_photon(general, photons):
     for g in got:
         # the instantiations of the general kernel contract differently: a path may part from another's
         assert g[1] == photons and abs(g[2] - got[0][2]) <= 2e-3 * photons ** 0.5 * 10 and abs(g[3] / got[0][3] - 1) <= 0.02
+
+
+_TWICE = '''
+import ctypes, sys
+sys.path[:0] = [%r, %r]
+import numpy as np, cases
+from mcxcl_gb300 import _lib, pmcxcl
+L, C = _lib.load(), _lib.Config()
+cfg = cases.small_two_media(nphoton=2000, savedetflag="dsp", prop=[[0, 0, 1, 1]] + [[0.01, 1, 0.5, 1.37]] * %d, **%r)
+pmcxcl.parse_config(cfg, C)
+L.mcx_validatecfg(ctypes.byref(C), None, None, 0)
+s = L.mcx_prepare_simulation(ctypes.byref(C))
+pmcxcl._check(C)
+for _ in range(2):
+    assert L.mcxg_set_launch(s, 256, 4) == 0 and L.mcxg_simulate(s, 2, ctypes.byref(ctypes.c_float())) == 0
+    g = ctypes.c_int()
+    L.mcxg_get_launch(s, ctypes.byref(g), None, None)
+    print(g.value)
+'''
+
+
+@pytest.mark.parametrize("media,extra,blocks", [(30, {}, 3), (60, {}, 1), (30, dict(gscatter=1 << 24), 3)])
+def test_no_more_blocks_than_fit(media, extra, blocks):
+    """Records of many media leave room for fewer blocks a SM (their shared memory: 2 x 1 KB a medium and block of 228 KB),
+    in a process's first launch of a kernel as in its second."""
+    import os
+    import subprocess
+    import sys
+
+    import mcxcl_gb300
+    here = os.path.dirname(os.path.abspath(__file__))
+    p = subprocess.run([sys.executable, "-c", _TWICE % (os.path.dirname(here), here, media, extra)], capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0, p.stderr[-2000:]
+    sms = mcxcl_gb300.gpuinfo()[0]["sm"]
+    assert [int(x) // sms for x in p.stdout.split()] == [blocks, blocks]
