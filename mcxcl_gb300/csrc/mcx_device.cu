@@ -577,11 +577,17 @@ size_t shared_bytes(const mcxg_kparams& kp, int block) {
    them measured the same on the three (shapes of 1 to 4 blocks x 2 to 32
    lanes, 3e3 to 2e7 photons).  The other kernels, with more instructions a
    step, gain from fewer warps only below 1,000 photons an SM (the replay of
-   9,000 photons 4.7 -> 3.7 ms); at 1e6 photons 2 blocks were 5 to 10 % slower
-   than 4. */
-int blocks_for(unsigned long long photons, int sms, bool label) {
+   9,000 photons 4.7 -> 3.7 ms; at 1e6 photons 2 blocks were 5 to 10 % slower
+   than 4), and two of them not that far: at 330 photons split voxels took 5 %
+   more with 1 block than with 3, half-precision labels 2 % more at 460 and 5 %
+   at 1,000; shared patterns 2 to 6 % more from 800 on. */
+unsigned long long few_photons(const mcxg_kparams& kp) {
+    return (kp.mediaformat > 4 && kp.mediaformat != 101) ? 300 : (kp.srcnum > 1 ? 700 : 1000);
+}
+
+int blocks_for(const mcxg_kparams& kp, unsigned long long photons, int sms, bool label) {
     const unsigned long long q = photons / (unsigned int)sms;
-    if (q <= 1000) {
+    if (q <= few_photons(kp)) {
         return q <= 96 ? 2 : 1;
     }
     return !label ? 4 : (q <= 10000 ? 2 : (q <= 35000 ? 3 : 4));
@@ -590,9 +596,9 @@ int blocks_for(unsigned long long photons, int sms, bool label) {
 /* Lanes of each warp that take work: one photon a lane as long as the warps
    that are resident have a lane for each.  Asked once the blocks are known, a
    caller's own and what shared memory leaves of them included. */
-unsigned int lanes_for(unsigned long long photons, int sms, int warps) {
+unsigned int lanes_for(const mcxg_kparams& kp, unsigned long long photons, int sms, int warps) {
     const unsigned long long q = photons / (unsigned int)sms;
-    return (unsigned int)std::min(32ull, std::max(1ull, (q + warps - 1) / warps));
+    return q > few_photons(kp) ? 32u : (unsigned int)std::min(32ull, std::max(1ull, (q + warps - 1) / warps));
 }
 
 /* What mcx_transport_label does for a run (RUN_FWD ..), or -1: it takes 3-D
@@ -1642,7 +1648,7 @@ int mcxg_simulate(mcxg_session* s, unsigned int flags, float* kernel_ms) {
     int bpsm = exact ? 2 : bpsm_sel;
     const unsigned long long photons = (unsigned long long)kp.threadphoton * kp.nthread + (unsigned long long)std::max(kp.oddphoton, 0);
     if (!exact && adjmode != 2u && !s->block_req && !s->bpsm_req) {
-        bpsm = std::min(bpsm, blocks_for(photons, s->info.sm, label));
+        bpsm = std::min(bpsm, blocks_for(kp, photons, s->info.sm, label));
     }
     if (!exact) {
         /* never more blocks than fit at once: a persistent grid must be resident */
@@ -1655,7 +1661,7 @@ int mcxg_simulate(mcxg_session* s, unsigned int flags, float* kernel_ms) {
     if (bpsm < 1) {
         bpsm = 1;
     }
-    a.lanes = (exact || adjmode == 2u) ? 32u : lanes_for(photons, s->info.sm, bpsm * block / 32);
+    a.lanes = (exact || adjmode == 2u) ? 32u : lanes_for(kp, photons, s->info.sm, bpsm * block / 32);
     s->lanes = (int)a.lanes;
     int grid = s->info.sm * bpsm;
     s->grid = grid;
@@ -1719,7 +1725,7 @@ int mcxg_autotune(mcxg_session* s, uint32_t sample_photons, int* block, int* blo
        configurations' kernel has no other shape of 256 threads, its blocks having
        one register budget */
     const bool label = !s->tile_req && usual_run(s, full, 0u, mcxg::kLabelBlock) >= 0;
-    cands[0].bpsm = blocks_for(total, s->info.sm, label);
+    cands[0].bpsm = blocks_for(full, total, s->info.sm, label);
     float best = 1e30f;
     Cand pick = cands[0];
     int keep_block = s->block_req, keep_bpsm = s->bpsm_req;

@@ -199,3 +199,16 @@ def test_no_more_blocks_than_fit(media, extra, blocks):
     assert p.returncode == 0, p.stderr[-2000:]
     sms = mcxcl_gb300.gpuinfo()[0]["sm"]
     assert [int(x) // sms for x in p.stdout.split()] == [blocks, blocks]
+
+
+def test_where_few_photons_end():
+    """Other media formats and shared patterns, which gain less from few warps, take their full shape earlier."""
+    import mcxcl_gb300
+    L, s = _session()
+    sms = mcxcl_gb300.gpuinfo()[0]["sm"]
+    for variant, line, full in (("asf2h", 300, 3), ("svmc", 300, 3), ("pattern_share", 700, 4), ("gscatter", 1000, 4), ("angleinvcdf", 1000, 2)):
+        cfg = cases.small_two_media(**dict(cases.VARIANTS[variant], issaveseed=0))
+        for photons, blocks in ((line * sms, 1), ((line + 1) * sms, full)):
+            mcxcl_gb300.run(dict(cfg, nphoton=photons))
+            assert _launch(L, s) == (blocks * sms, 256)
+            assert _kernel(L, s)[1] == (min(32, -(-line // 8)) if blocks == 1 else 32)
