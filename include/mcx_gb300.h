@@ -404,7 +404,8 @@ int  mcxg_destroy(mcxg_session* s);
  * mediaword bytes each (1: label | detector bit << 7; 4: the reference's
  * 32-bit word), or with mediaword MCXG_MEDIA_PACK the reference's 32-bit
  * words (label | detector bit 31, labels below 128, medianum <= 128), which
- * the device packs to the one-byte form.  prop: medianum x 4 floats; detpos: detnum x 4; srcextra:
+ * the device packs to the one-byte form.  In the one-byte form a label past the
+ * last medium is taken as the last.  prop: medianum x 4 floats; detpos: detnum x 4; srcextra:
  * extrasrclen x 16; tables may be NULL when their length is 0.
  */
 int  mcxg_set_problem(mcxg_session* s, const void* kparams, size_t kparams_size, const void* media,
@@ -462,7 +463,8 @@ int  mcxg_get_tile(mcxg_session* s, uint32_t* box);
    bit << 7) and field.  Reference threads are numbered contiguously across
    the batch (vt_off); seeds come from splitmix64 of the simulation's seed.
    The simulations run in waves of 136, whose descriptors the kernel reads
-   from constant memory.  Not supported in a batch: detectors, replay, extra
+   from constant memory.  A label past a simulation's last medium is taken as
+   the last.  Not supported in a batch: detectors, replay, extra
    sources, patterns, phase tables, encodings other than labels. */
 int  mcxg_batch_set(mcxg_session* s, const void* sims, size_t desc_size, uint32_t nsim, const uint8_t* media,
                     uint64_t nmedia);

@@ -971,9 +971,9 @@ int mcxg_destroy(mcxg_session* s) {
 
 namespace {
 /* 32-bit label words (label | detector bit 31) to the kernel's bytes (label |
-   detector bit 7, the bits of keep), labels below 128; bounded by the last
-   medium, which the transport kernel's tables and record slots rely on (the
-   host driver has refused larger ones before) */
+   detector bit 7, the bits of keep), labels below 128; bounded by `last`, the
+   last medium or row of a batch, which the transport kernel's tables and record
+   slots rely on (the host driver has refused larger ones before) */
 __global__ void pack_labels(const uint32_t* __restrict__ words, size_t n, uint32_t keep, uint32_t last,
                             uint8_t* __restrict__ bytes) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
@@ -2297,7 +2297,16 @@ int batch_upload(mcxg_session* s, const mcxg_simdesc* sims, uint32_t nsim, const
     if (rc) {
         return rc;
     }
-    MCXG_TRY(cudaMemcpyAsync(s->d_sims, sims, sizeof(mcxg_simdesc) * nsim, cudaMemcpyHostToDevice, s->st));
+    /* labels are bounded by the last of MCXG_BATCH_MAXMEDIA rows: the rows past a simulation's own media
+       repeat its last one (a row of zeros is a medium of infinite 1/mus, in which a photon never ends).  The
+       volume itself is not rewritten by simulation, as simulations may share one */
+    std::vector<mcxg_simdesc> own(sims, sims + nsim);
+    for (mcxg_simdesc& d : own) {
+        for (uint32_t m = std::max(d.kp.medianum, 1u); m < MCXG_BATCH_MAXMEDIA; m++) {
+            d.prop[m] = d.prop[m - 1];
+        }
+    }
+    MCXG_TRY(cudaMemcpyAsync(s->d_sims, own.data(), sizeof(mcxg_simdesc) * nsim, cudaMemcpyHostToDevice, s->st));
     MCXG_TRY(cudaMemcpyAsync(s->d_simvt, simvt.data(), sizeof(unsigned long long) * (nsim + 1), cudaMemcpyHostToDevice,
                              s->st));
     if (words) {
@@ -2318,7 +2327,7 @@ int batch_upload(mcxg_session* s, const mcxg_simdesc* sims, uint32_t nsim, const
     batch_recip<<<grid_for(s, (size_t)nsim * MCXG_BATCH_MAXMEDIA), 256, 0, s->st>>>(s->d_sims, nsim);
     MCXG_TRY(cudaStreamSynchronize(s->st));
     MCXG_TRY(cudaGetLastError());
-    s->h_sims.assign(sims, sims + nsim);
+    s->h_sims = std::move(own);
     s->h_simvt = simvt;
     s->nsim = nsim;
     s->totalvt = vt;

@@ -212,3 +212,31 @@ def test_where_few_photons_end():
             mcxcl_gb300.run(dict(cfg, nphoton=photons))
             assert _launch(L, s) == (blocks * sms, 256)
             assert _kernel(L, s)[1] == (min(32, -(-line // 8)) if blocks == 1 else 32)
+
+
+@pytest.mark.parametrize("general", [{}, dict(gscatter=1 << 24)])
+def test_batch_labels_past_the_last_medium(general):
+    """A caller of the C interface may hand in a volume that validation has not seen: labels past a simulation's media
+    are its last medium, not another simulation's or an empty row."""
+    from mcxcl_gb300 import _lib, pmcxcl
+    L, got = _lib.load(), []
+    one, two = [[0, 0, 1, 1], [0.01, 1, 0.5, 1.37]], [[0, 0, 1, 1], [0.01, 1, 0.5, 1.37], [0.02, 5, 0.9, 1.45]]
+    for past in (False, True):
+        Cs = [_lib.Config() for _ in range(4)]
+        try:
+            for k, C in enumerate(Cs):
+                pmcxcl.parse_config(_plain(nphoton=3000, seed=k + 1, prop=two if k % 2 else one,
+                                           vol=np.full((20, 20, 20), 1 + k % 2, np.uint8), srcpos=[10, 10, 0], **general), C)
+                L.mcx_validatecfg(ctypes.byref(C), None, None, 0)
+                pmcxcl._check(C)
+                if past:
+                    np.ctypeslib.as_array(C.vol, shape=(8000,))[:] = (2, 3, 3, 120)[k]
+            L.mcx_run_batch((ctypes.POINTER(_lib.Config) * 4)(*[ctypes.pointer(C) for C in Cs]), 4, ctypes.c_uint(0), ctypes.c_uint(0))
+            pmcxcl._check(Cs[0])
+            got.append([(C.energytot, C.energyesc) + tuple(np.ctypeslib.as_array(C.exportfield, shape=(8000 * 20,)).tolist()) for C in Cs])
+        finally:
+            for C in Cs:
+                L.mcx_clearcfg(ctypes.byref(C))
+    for a, b in zip(*got):
+        assert a[:2] == b[:2] and 0 < a[1] < a[0] == 3000
+        assert np.abs(np.array(a[2:]) - np.array(b[2:])).max() <= 1e-6 * max(a[2:])
