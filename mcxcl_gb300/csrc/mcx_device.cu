@@ -361,19 +361,19 @@ __global__ void batch_recip(mcxg_simdesc* __restrict__ sims, unsigned int nsim) 
 }
 
 /* per-simulation FP64 energy sums, in an order fixed by the simulation's own
-   threads: row y of the grid is simulation y, its kEnergyParts blocks each sum a
-   stride of them (one block a simulation left 24 of 152 SMs, each with two FP64
+   threads: column x of the grid is simulation x (y ends at 65,535), its
+   kEnergyParts blocks each sum a stride of them (one block a simulation left 24 of 152 SMs, each with two FP64
    operations a cycle, to it: 0.54 ms for 2.3 M threads, 0.03 so), then
    batch_energy_final adds the parts */
 constexpr unsigned int kEnergyParts = 32;
 
 __global__ void __launch_bounds__(256) batch_energy(const float2* __restrict__ e, const mcxg_simdesc* __restrict__ sims,
                                                     double* __restrict__ part) {
-    const mcxg_simdesc& d = sims[blockIdx.y];
+    const mcxg_simdesc& d = sims[blockIdx.x];
     const unsigned long long base = d.vt_off;
     const unsigned int n = d.kp.nthread;
     double se = 0.0, sl = 0.0;
-    for (unsigned int i = blockIdx.x * 256u + threadIdx.x; i < n; i += kEnergyParts * 256u) {
+    for (unsigned int i = blockIdx.y * 256u + threadIdx.x; i < n; i += kEnergyParts * 256u) {
         float2 v = e[base + i];
         se += (double)v.x;
         sl += (double)v.y;
@@ -394,7 +394,7 @@ __global__ void __launch_bounds__(256) batch_energy(const float2* __restrict__ e
             a += wse[w];
             b += wsl[w];
         }
-        double* p = part + 2 * ((size_t)blockIdx.y * kEnergyParts + blockIdx.x);
+        double* p = part + 2 * ((size_t)blockIdx.x * kEnergyParts + blockIdx.y);
         p[0] = a;
         p[1] = b;
     }
@@ -2238,7 +2238,7 @@ int batch_enqueue(mcxg_session* s, int lflags) {
         MCXG_TRY(mcxg::batch_launch(a, lflags, s->bt_grid, s->bt_block, s->st));
     }
     double* part = s->d_bsum + 2 * (size_t)s->nsim;
-    batch_energy<<<dim3(kEnergyParts, s->nsim), 256, 0, s->st>>>(s->d_benergy, s->d_sims, part);
+    batch_energy<<<dim3(s->nsim, kEnergyParts), 256, 0, s->st>>>(s->d_benergy, s->d_sims, part);
     batch_energy_final<<<(2 * s->nsim + 255) / 256, 256, 0, s->st>>>(part, s->nsim, s->d_bsum);
     return MCXG_OK;
 }

@@ -240,3 +240,26 @@ def test_batch_labels_past_the_last_medium(general):
     for a, b in zip(*got):
         assert a[:2] == b[:2] and 0 < a[1] < a[0] == 3000
         assert np.abs(np.array(a[2:]) - np.array(b[2:])).max() <= 1e-6 * max(a[2:])
+
+
+def test_energies_of_more_simulations_than_a_grid_is_high():
+    """65,540 simulations of two photons: the batch runs and its energies are summed (its fields are read in a grid whose
+    second dimension ends at 65,535, so the call that wants them too refuses)."""
+    from mcxcl_gb300 import _lib, pmcxcl
+    L, s = _session()
+    cfg = dict(nphoton=2, vol=np.ones((2, 2, 2), np.uint8), prop=[[0, 0, 1, 1], [0.01, 1, 0.5, 1.37]], srcpos=[1, 1, 0], srcdir=[0, 0, 1],
+               issrcfrom0=1, tstart=0, tend=5e-9, tstep=5e-9, isreflect=0, issavedet=0, seed=3)
+    n = 65540
+    Cs = [_lib.Config() for _ in range(n)]
+    try:
+        for C in Cs:
+            pmcxcl.parse_config(cfg, C)
+            L.mcx_validatecfg(ctypes.byref(C), None, None, 0)
+        L.mcx_run_batch((ctypes.POINTER(_lib.Config) * n)(*[ctypes.pointer(C) for C in Cs]), n, ctypes.c_uint(0), ctypes.c_uint(0))
+        assert L.mcxg_batch_simulate(ctypes.c_void_p(s), ctypes.c_uint(0), ctypes.byref(ctypes.c_float())) == 0
+        e = np.zeros((n, 2))
+        assert L.mcxg_batch_get_energy(ctypes.c_void_p(s), ctypes.c_void_p(e.ctypes.data)) == 0
+    finally:
+        for C in Cs:
+            L.mcx_clearcfg(ctypes.byref(C))
+    assert (e[:, 1] == 2).all() and (e == e[0]).all() and 0 < e[0, 0] <= 2
