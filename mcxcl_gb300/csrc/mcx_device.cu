@@ -650,12 +650,14 @@ size_t label_shared_bytes(const mcxg_kparams& kp) {
    starts out of step and its order varies more (two calls' dL/dmus 5.7e-6 apart
    on average, 3.7 to 4.1e-6 with its own kernel before it; 1e6 photons, 60^3). */
 int usual_run(const mcxg_session* s, const mcxg_kparams& kp, unsigned int flags, int block) {
-    if ((flags & (MCXG_EXACT | MCXG_RNGDUMP | MCXG_GENERAL | MCXG_VERIFY | MCXG_ADJ1 | MCXG_ADJ2)) || s->npol || s->maxjump ||
+    if ((flags & (MCXG_EXACT | MCXG_RNGDUMP | MCXG_GENERAL | MCXG_ADJ1 | MCXG_ADJ2)) || s->npol || s->maxjump ||
             block != mcxg::kLabelBlock) {
         return -1;
     }
     /* a slot more for each kind of record: the last media that fit the other kernel's layout */
-    return label_shared_bytes(kp) > s->info.sharedmem_per_block ? -1 : label_run(kp);
+    const int run = label_shared_bytes(kp) > s->info.sharedmem_per_block ? -1 : label_run(kp);
+    /* the precision check vouches for the kernel that the run without it takes */
+    return (flags & MCXG_VERIFY) ? (run == mcxg::RUN_FWD && kp.mediaformat <= 4 ? mcxg::RUN_CHECK : -1) : run;
 }
 
 /* q = umulhi(n, m) >> sh equals n / d for every n < bound: m = ceil(2^(32+sh) / d)
@@ -2393,7 +2395,7 @@ int mcxg_batch_simulate(mcxg_session* s, unsigned int flags, float* kernel_ms) {
     int lflags = (refl ? mcxg::LF_REFL : 0) | (agg ? mcxg::LF_WAGG : 0) | (bpsm_req >= 3 ? mcxg::LF_CAPPED : 0) |
                  (common && !(flags & MCXG_GENERAL) ? mcxg::LF_COMMON : 0) | (verify ? mcxg::LF_ACC64 : 0);
     const int block = s->block_req ? s->block_req : 256;
-    if (label && !agg && !verify && !(flags & MCXG_GENERAL) && block == mcxg::kLabelBlock) {
+    if (label && !agg && !(flags & MCXG_GENERAL) && block == mcxg::kLabelBlock) {
         lflags |= mcxg::LF_LABEL;
     }
     s->usual = (lflags & mcxg::LF_LABEL) != 0;

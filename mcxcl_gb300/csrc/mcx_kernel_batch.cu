@@ -47,6 +47,10 @@ static void* kbatch_acc64() {
 
 static void* select(int flags) {
     const bool refl = flags & LF_REFL, wagg = flags & LF_WAGG, cap = flags & LF_CAPPED;
+    if ((flags & LF_LABEL) && (flags & LF_ACC64)) {
+        return refl ? (void*)mcx_transport_label<RUN_CHECK, VOL_LABEL, DET_NONE, true>
+                    : (void*)mcx_transport_label<RUN_CHECK, VOL_LABEL, DET_NONE, false>;
+    }
     if (flags & LF_LABEL) {
         return refl ? (void*)mcx_transport_label<RUN_FWD, VOL_LABEL, DET_NONE, true>
                     : (void*)mcx_transport_label<RUN_FWD, VOL_LABEL, DET_NONE, false>;

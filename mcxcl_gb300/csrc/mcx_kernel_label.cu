@@ -30,7 +30,7 @@ static void* krefl(int flags) {
     return (flags & LF_REFL) ? (void*)mcx_transport_label<KIND, VOL, DET, true> : (void*)mcx_transport_label<KIND, VOL, DET, false>;
 }
 
-/* the replays, the RF run: records of any kind or none */
+/* the replays, the RF run, the precision check: records of any kind or none */
 template <int KIND, int VOL>
 static void* kany(int flags) {
     return (flags & LF_DET) ? krefl<KIND, VOL, DET_ANY>(flags) : krefl<KIND, VOL, DET_NONE>(flags);
@@ -60,6 +60,9 @@ static void* kvol(int flags) {
 static void* select(int flags) {
     if ((flags >> LF_RUN & 0xF) == RUN_RF) {
         return kany<RUN_RF, VOL_LABEL>(flags);
+    }
+    if ((flags >> LF_RUN & 0xF) == RUN_CHECK) {
+        return kany<RUN_CHECK, VOL_LABEL>(flags);
     }
     return (flags & LF_MUA) ? kvol<VOL_MUA>(flags) : kvol<VOL_LABEL>(flags);
 }

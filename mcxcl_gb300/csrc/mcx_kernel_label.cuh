@@ -2,8 +2,8 @@
  * mcx_kernel_label.cuh -- the transport kernel of the usual configurations.
  *
  * Byte labels or float absorption, three dimensions, Henyey-Greenstein, one
- * source; deposits of flux, fluence or energy, replays and modulated sources
- * -- each with all of that fixed at compile time.  The photons, their random numbers and every
+ * source; deposits of flux, fluence or energy, their precision check, replays
+ * and modulated sources -- each with all of that fixed at compile time.  The photons, their random numbers and every
  * rounding are those of mcx_transport (mcx_kernel.cuh), whose device
  * functions it shares; what differs is what a step costs.
  *
@@ -418,7 +418,7 @@ __device__ __forceinline__ void startbeam(const PS& ps, Photon& s) {
 }
 
 template <int KIND, int VOL, int DET, bool REFL>
-__global__ void __launch_bounds__(LB_BLOCK, KIND == RUN_RF ? 3 : 4) mcx_transport_label(const KArgs a) {
+__global__ void __launch_bounds__(LB_BLOCK, KIND == RUN_RF || KIND == RUN_CHECK ? 3 : 4) mcx_transport_label(const KArgs a) {
     typedef Mth<false> M;
     typedef Voxel<VOL> V;
     constexpr bool GEN = VOL == VOL_MUA || KIND == RUN_RF;
@@ -643,6 +643,9 @@ __global__ void __launch_bounds__(LB_BLOCK, KIND == RUN_RF ? 3 : 4) mcx_transpor
                         atomicAdd(a.fhi + key, (unsigned long long)__float2ll_rn(kf));
                         if (r != 0.f) {
                             atomicAdd(a.flo + key, r);
+                        }
+                        if (KIND == RUN_CHECK) {
+                            acc_verify(a, ps.lo_plane(), key, weight);
                         }
                     }
                 }

@@ -90,7 +90,7 @@ struct KArgs {
 enum { LF_DET = 1, LF_REFL = 2, LF_WAGG = 4, LF_CAPPED = 8, LF_XMEDIA = 32, LF_COMMON = 64, LF_RF = 128, LF_POL = 256, LF_SVMC = 512,
        LF_ACC64 = 1024, LF_ADJ = 2048, LF_TILE = 4096,
        /* for the label kernel: float absorption; bit positions of what the run
-          does (RUN_FWD .. RUN_RF) and of savedetflag's partial-data bits */
+          does (RUN_FWD .. RUN_CHECK) and of savedetflag's partial-data bits */
        LF_MUA = 8192, LF_RUN = 16, LF_KINDS = 20,
        LF_LABEL = 1 << 24 /* batches: that kernel */ };
 
@@ -106,7 +106,8 @@ enum {
     RUN_FWD,    /* deposits flux, fluence or energy */
     RUN_JAC,    /* replay: the detected weight (x time of flight) times the path in each voxel */
     RUN_SITE,   /* replay: the detected weight (x time of flight, x 1 - cos theta) at each scattering */
-    RUN_RF      /* modulated source: complex weight and field */
+    RUN_RF,     /* modulated source: complex weight and field */
+    RUN_CHECK   /* RUN_FWD with every deposit also in an FP64, a float and a spill field */
 };
 
 constexpr int kLabelBlock = 256;   /* its threads a block */

@@ -263,3 +263,37 @@ def test_energies_of_more_simulations_than_a_grid_is_high():
         for C in Cs:
             L.mcx_clearcfg(ctypes.byref(C))
     assert (e[:, 1] == 2).all() and (e == e[0]).all() and 0 < e[0, 0] <= 2
+
+
+def test_the_precision_check_runs_the_kernel_it_vouches_for():
+    import mcxcl_gb300
+    from mcxcl_gb300 import _lib, pmcxcl
+    L, C = _lib.load(), _lib.Config()
+    for cfg, usual in ((_plain(nphoton=20000), 1), (cases.small_two_media(nphoton=20000), 1), (_plain(nphoton=20000, isreflect=0), 1),
+                       (_plain(nphoton=20000, gscatter=1 << 24), 0)):
+        try:
+            pmcxcl.parse_config(cfg, C)
+            L.mcx_validatecfg(ctypes.byref(C), None, None, 0)
+            s = L.mcx_prepare_simulation(ctypes.byref(C))
+            pmcxcl._check(C)
+            fields = []
+            for flags in (2, 2 | 128):
+                assert L.mcxg_simulate(s, flags, ctypes.byref(ctypes.c_float())) == 0
+                assert _usual(L, s) == usual
+                fields.append(np.zeros(40 ** 3 * 20))
+                assert L.mcxg_get_field_f64(s, fields[-1].ctypes.data) == 0
+            f64, plain, spill = np.zeros(fields[0].size), np.zeros(fields[0].size, np.float32), np.zeros(fields[0].size, np.float32)
+            assert L.mcxg_get_verify(s, f64.ctypes.data, plain.ctypes.data, spill.ctypes.data) == 0
+        finally:
+            L.mcx_clearcfg(ctypes.byref(C))
+        # the same photons as without the check, to the field's rounded remainders; the general kernel's instantiations
+        # contract differently.  Plain sums of 2e4 terms of one sign are off by at most 2e4 half ulps, 1.2e-3 (the spill
+        # field loses what two additions at once both carry over: it is what the others are measured against, not checked)
+        norm = np.linalg.norm(f64)
+        assert norm > 0 and np.linalg.norm(fields[1] - f64) <= 1e-6 * norm
+        assert not usual or np.linalg.norm(fields[0] - f64) <= 1e-6 * norm
+        assert np.linalg.norm(plain - f64) <= 1.2e-3 * norm and spill.any()
+    sims = [_plain(nphoton=3000, seed=k + 1) for k in range(3)]
+    for extra, usual in (({}, 1), (dict(gscatter=1 << 24), 0)):
+        got = mcxcl_gb300.run_batch([dict(c, **extra) for c in sims], verify=True)
+        assert _usual(L, s) == usual and max(o["stat"]["relerr_max"] for o in got) < 1e-6
