@@ -1275,6 +1275,11 @@ int mcx_rand_blocks(unsigned int seed, uint64_t skip, uint32_t nblock, uint32_t 
     return 0;
 }
 
+/* a fourierx source's largest weight for its modulation parameter (1 in [0, 2]) */
+static double fourierx_weight(float w) {
+    return fmax(1.0, 0.5 * (fabs(1.0 - (double)w) + 1.0));
+}
+
 /* The field accumulator's fixed-point unit 2^-S (the transport kernel's
    deposits split into int64 counts of 2^-S and float remainders): the
    largest S, at most 40, for which no element can reach 2^62 counts.  An
@@ -1299,9 +1304,10 @@ static void field_scale(const Config* cfg, int replay, float* sc, float* unit) {
     }
     double each = 4.0 * path * wmax;
     if (!replay && cfg->mediabyte <= 4 && !(cfg->omega > 0.f) && !(cfg->minenergy > 0.f) && cfg->outputtype != otL) {
-        double loss = fabs((double)cfg->srcpos.w);
+        const int fourierx = cfg->srctype == MCX_SRC_FOURIERX;
+        double loss = fabs((double)cfg->srcpos.w) * (fourierx ? fourierx_weight(cfg->srcparam2.w) : 1.0);
         for (unsigned int i = 0; i < cfg->extrasrclen; i++) {
-            loss = fmax(loss, fabs((double)cfg->srcdata[i].srcpos.w));
+            loss = fmax(loss, fabs((double)cfg->srcdata[i].srcpos.w) * (fourierx ? fourierx_weight(cfg->srcdata[i].srcparam2.w) : 1.0));
         }
         if (cfg->srctype == MCX_SRC_PATTERN || cfg->srctype == MCX_SRC_PATTERN3D) {
             loss = INFINITY;             /* the pattern's values scale the weight: the path bound stands */

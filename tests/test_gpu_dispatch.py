@@ -297,3 +297,17 @@ def test_the_precision_check_runs_the_kernel_it_vouches_for():
     for extra, usual in (({}, 1), (dict(gscatter=1 << 24), 0)):
         got = mcxcl_gb300.run_batch([dict(c, **extra) for c in sims], verify=True)
         assert _usual(L, s) == usual and max(o["stat"]["relerr_max"] for o in got) < 1e-6
+
+
+@pytest.mark.parametrize("depth", [0.5, -9, -1000])
+def test_weights_above_one_stay_within_the_fields_range(depth):
+    """A fourierx source's weight grows with its modulation parameter: 501 at -1000.  What the field holds is what the
+    photons left, to the roundings of weights (some 20 steps of 6e-8)."""
+    import mcxcl_gb300
+    cfg = dict(nphoton=1000000, vol=np.ones((6, 6, 6), np.uint8), prop=[[0, 0, 1, 1], [1.0, 1, 0.5, 1]], srcpos=[2, 2, 0],
+               srctype="fourierx", srcdir=[0, 0, 1], srcparam1=[1, 0, 0, 1], srcparam2=[0, 0, 0, depth], issrcfrom0=1, seed=5,
+               tstart=0, tend=5e-9, tstep=5e-9, isreflect=0, issavedet=0, outputtype="energy", isnormalized=0)
+    r = mcxcl_gb300.run(cfg)
+    tot, esc = r["stat"]["energytot"], r["stat"]["energyesc"]
+    assert abs(tot / (1e6 * (2 - depth) / 2) - 1) < 1e-4
+    assert abs(np.asarray(r["flux"], np.float64).sum() / (tot - esc) - 1) < 1e-5
