@@ -1286,7 +1286,7 @@ static double fourierx_weight(float w) {
    element gathers at most every photon's whole path -- the time window at
    the speed of light, in voxels -- times its weight (a replay: the largest
    replay weight), with a factor 4 to spare.  Where photons only lose weight
-   (labels, real weights, no roulette) a photon also leaves no more than its
+   (labels, real weights, no roulette, no negative mua) a photon also leaves no more than its
    launch weight as energy, or that over the least mua as flux, in all
    elements together (a factor 2 to spare).  The larger S is worth having: a
    deposit of 2^(23-S) or more is a whole number of units, so its remainder
@@ -1317,8 +1317,9 @@ static void field_scale(const Config* cfg, int replay, float* sc, float* unit) {
         for (unsigned int i = 1; i < cfg->medianum; i++) {
             mua = fmin(mua, (double)cfg->prop[i].mua);
         }
-        /* the saved reflectance deposits the weight itself */
-        const double most = cfg->outputtype == otEnergy ? loss : (mua > 0.0 ? loss * fmax(1.0, 1.0 / mua) : INFINITY);
+        /* the saved reflectance deposits the weight itself; a medium of negative mua adds weight */
+        const double most = mua < 0.0 ? INFINITY : (cfg->outputtype == otEnergy ? loss
+                            : (mua > 0.0 ? loss * fmax(1.0, 1.0 / mua) : INFINITY));
         each = fmin(each, 2.0 * most);
     }
     const double bound = (double)(cfg->nphoton ? cfg->nphoton : 1) * each;
