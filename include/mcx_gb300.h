@@ -436,7 +436,8 @@ int  mcxg_get_seeds(mcxg_session* s, uint32_t* out, uint32_t nthread);
 int  mcxg_set_trajectory(mcxg_session* s, uint32_t maxrec);
 int  mcxg_get_trajectory(mcxg_session* s, float* out, uint32_t maxrec, uint32_t* count);
 /* Launch shape of the persistent grid: block threads (32..256, a multiple of
-   32) and resident blocks per SM (0 = automatic: 256 threads x 4).  Shapes of
+   32) and resident blocks per SM (0, 0 = automatic: 256 threads, 1 to 4 blocks by
+   the photons per SM).  Shapes of
    more than 512 threads per SM run the instantiation whose registers are
    capped for 1,024 resident threads (64 a thread; the specialised RF,
    polarised, split-voxel, other-encoding, precision-check and gradient
@@ -494,9 +495,9 @@ int  mcxg_batch_get_field(mcxg_session* s, float* out, const double* scales);
 int  mcxg_set_replay(mcxg_session* s, const void* seeds16, const float* weight, const float* tof, const int* detid,
                      uint32_t n);
 /* Pick the launch shape of the fast kernel for the current problem: time
-   each candidate (blocks of 256, 128 and 64 threads at 1,024 resident
-   threads per SM with capped registers, 256 and 128 at 512 with uncapped
-   ones; then
+   each candidate (blocks of 256 threads as many a SM as the automatic shape
+   has, 128 and 64 at 1,024 resident threads per SM with capped registers, 128
+   and, for the general kernel, 256 at 512 with uncapped ones; then
    the fastest with warp-aggregated deposits) on the first sample_photons
    photons and keep the fastest for later mcxg_simulate calls (unless a
    shape was set with mcxg_set_launch).  Outputs may be NULL.  The trial

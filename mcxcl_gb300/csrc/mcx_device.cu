@@ -567,7 +567,7 @@ size_t shared_bytes(const mcxg_kparams& kp, int block) {
 /* Blocks per SM (of 256 threads) for a run of `photons`, and lanes per warp.
    A photon takes up to thousands of steps one after another, so a run cannot
    end before its longest photon, and a step takes the longer the more warps
-   share the SM (cube: 3 us at 32 warps, 0.55 us at a few) and the more lanes
+   share the SM (cube: 3 us at 32 warps, 0.45 us at a few) and the more lanes
    of the warp go different ways.  A large run wants all the warps for
    throughput; one with few photons per SM is faster with fewer.  Kernel times
    in ms at 4 blocks x 32 lanes and as here: cube 1e4 photons 2.01 -> 1.20,
@@ -1179,7 +1179,7 @@ __global__ void __launch_bounds__(128) lfib_words(const uint32_t* __restrict__ s
    b >= 5 of its first block's index, then by Q_0 from one block's window to the
    next; each lane then expands one of the windows as lfib_words does.  (A
    thread for each block did its 31 x 31 products alone: 151 us for 622,592
-   reference threads' words in blocks of 1,024, 15 us so in blocks of 124.) */
+   reference threads' words in blocks of 1,024, 22 us so in blocks of 124.) */
 __device__ __forceinline__ void lf_mul_shared(const uint32_t* X, const uint32_t* Y, uint32_t* Z, int t) {
     uint32_t acc = 0;
     if (t < 31 * 31) {
@@ -1585,7 +1585,7 @@ int mcxg_simulate(mcxg_session* s, unsigned int flags, float* kernel_ms) {
                  (common ? mcxg::LF_COMMON : 0) | (rf ? mcxg::LF_RF : 0) | (pol ? mcxg::LF_POL : 0) |
                  (svmc ? mcxg::LF_SVMC : 0) | (verify ? mcxg::LF_ACC64 : 0) | (adjmode ? mcxg::LF_ADJ : 0);
     if (verify) {
-        /* the precision check runs the fast common-configuration instantiation */
+        /* the precision check is a case of the common configuration */
         if (exact || !common || kp.replay || (flags & MCXG_KEEP)) {
             return MCXG_ERR_ARG;
         }

@@ -1,7 +1,7 @@
 /*
  * mcx_launch.h -- internal interface between the session code (mcx_device.cu)
- * and the two kernel translation units.  Each unit owns its own copy of the
- * constant block, so each exports its own upload and launch entry.
+ * and the four kernel translation units (fast, exact, label, batch).  Each owns its
+ * own copy of the constant block, so each exports its own upload and launch entry.
  */
 #ifndef MCX_LAUNCH_H
 #define MCX_LAUNCH_H
